@@ -356,3 +356,83 @@ def tolerance(case):
     if case["op"] == "obs":                                # scores and weights are rounded to the inputs' type
         return {"rel": 1e-4, "max": 4e-3} if case["dtype"] == "fp16" else {"rel": 1.4e-3, "max": 3e-2}
     return "exact"                                         # packed bytes, parameters, bit choices, fp16 rows
+
+
+# ── the same results in 64 bits ──────────────────────────────────────────────
+
+def _codes(packed, bits):
+    """Codes of packed rows [..., bytes] -> [..., bytes * 8 / bits]: part i of the columns holds the bits
+    from i * bits on of every byte."""
+    return torch.cat([(packed >> (bits * i)) & (2 ** bits - 1) for i in range(8 // bits)], dim=-1).double()
+
+
+def _dense(layer, v16, gqa):
+    """[(keys [n, 128], values [n, 128])] of the layer's heads, live rows only, from its packed bytes."""
+    heads, T_v = layer.K_ch_scale.shape[1], layer.T_eff
+    parts = [_codes(t[0], b) for t, b in ((layer.K_2bit, 2), (layer.K_4bit, 4), (layer.K_8bit, 8)) if t is not None]
+    slots = (torch.cat(parts, dim=-1) - layer.K_ch_zp[0].double()) * layer.K_ch_scale[0].double()
+    out = []
+    for h, ((n2, n4, n8), n16) in enumerate(zip(layer.seg_bounds_per_head.tolist(), layer.n_v16_per_head.tolist())):
+        keys = torch.zeros(slots.shape[1], D, dtype=torch.float64, device=DEV)
+        keys.index_add_(1, layer.K_ch_perm_padded_idx_for_Q[h * gqa], slots[h])
+        n = n2 + n4 + n8
+        rows = [_codes(t[0, h, :m], b) for t, m, b in ((layer.V_2bit, n2, 2), (layer.V_4bit, n4, 4), (layer.V_8bit, n8, 8)) if m]
+        values = (torch.cat(rows) - layer.V_zp[0, h, :n].double()) * layer.V_scale[0, h, :n].double() if rows else keys[:0]
+        if n16:
+            values = torch.cat([values, v16[0, h, :n16].double()])
+        out.append((torch.cat([keys[:n], keys[T_v:T_v + n16]]), values))
+    return out
+
+
+def _rotated(x, cos, sin):
+    lo, hi = x[..., :D // 2], x[..., D // 2:]
+    return torch.cat([lo * cos - hi * sin, hi * cos + lo * sin], dim=-1)
+
+
+def _exact_decode(s, gqa):
+    table, q = s["table"], s["q"].to(DEV).double()
+    out = torch.empty(q.shape, dtype=torch.float64, device=DEV)
+    for i, (layer, v16) in enumerate(table.source):
+        qi = q[i]
+        if "rope" in s:
+            cos, sin = (t[i].double() for t in s["rope"])
+            qi, k_cur = _rotated(qi, cos, sin), _rotated(s["k_cur"][i].double(), cos, sin)
+            n_new = int(s["n_new"]) if not torch.is_tensor(s["n_new"]) else int(s["n_new"][i])
+        for h, (keys, values) in enumerate(_dense(layer, v16, gqa)):
+            if "rope" in s:
+                keys = torch.cat([keys, s["new_k"][i, h, :n_new].double(), k_cur[h:h + 1]])
+                values = torch.cat([values, s["new_v"][i, h, :n_new].double(), s["v_cur"][i, h:h + 1].double()])
+            at = slice(h * gqa, (h + 1) * gqa)
+            out[i, at] = torch.softmax(qi[at] @ keys.T / D ** 0.5, dim=-1) @ values
+    return out
+
+
+def exact(case, seed):
+    """What ``run`` returns for ``prepare(case, seed)``, from the packed bytes (decode) or the inputs (scores) in
+    64 bits; None where the outputs are whole numbers, bytes and the fp16 parameters that go with them."""
+    op, gqa = case["op"], case.get("gqa")
+    if op not in ("block", "step", "host", "two_stage", "obs"):
+        return None
+    s = prepare(case, seed)
+    if op == "obs":
+        q, k = s["q"].double(), s["k"].double()
+        heads, W, T = k.shape[1], q.shape[2], k.shape[2]
+        token = torch.empty(1, heads, T, dtype=torch.float64, device=DEV)
+        unseen = torch.arange(T, device=DEV) > (T - W + torch.arange(W, device=DEV))[:, None]
+        for h in range(heads):
+            scores = (q[0, h * gqa:(h + 1) * gqa] @ k[0, h].T / D ** 0.5).masked_fill(unseen, float("-inf"))
+            token[0, h] = torch.softmax(scores, dim=-1).sum(dim=(0, 1)) / (~unseen).sum(dim=0)
+        channel = q.reshape(1, heads, -1, D).square().mean(dim=2) * k.square().mean(dim=2)
+        return token, channel
+    if op == "two_stage":
+        layer, T_v = s["layer"], s["layer"].T_eff
+        weights = torch.zeros(s["scores"].shape, dtype=torch.float64, device=DEV)
+        out = torch.empty(s["out"].shape, dtype=torch.float64, device=DEV)
+        for h, (keys, values) in enumerate(_dense(layer, None if s["v16"] is None else s["v16"][None], gqa)):
+            at, n = slice(h * gqa, (h + 1) * gqa), int(layer.seg_bounds_per_head[h].sum())
+            w = torch.softmax(s["q"][at].double() @ keys.T / D ** 0.5, dim=-1)
+            weights[at, :n], weights[at, T_v:T_v + w.shape[1] - n] = w[:, :n], w[:, n:]
+            out[at] = w @ values
+        return weights, out
+    out = _exact_decode(s, gqa)
+    return (out, None, None) if op == "block" else out
