@@ -37,6 +37,11 @@ enum { RDKV_F16 = 0, RDKV_BF16 = 1, RDKV_F32 = 2 };
  * [1]=l (sum of exp), [2..3]=0, [4..131]=o (un-normalised output, 128 channels) */
 #define RDKV_PARTIAL_STRIDE 132
 
+/* Added to the k_row_bytes_max argument of the decode entry points: K rows of any number of bytes at any
+ * address are expected (odd padded channel counts, more than one span of 16, 32 or 32 channels of 8, 4 or
+ * 2 bits), so the kernel that is fast for those is launched.  Results do not depend on it beyond rounding. */
+#define RDKV_K_ANY_ROWS 65536
+
 /*
  * One (sequence, layer) of packed cache: H_kv heads in the reference's stacked
  * per-head layout (PackedKVLayer, obkv_accel/packing.py:43-111, plus the fp16

@@ -33,6 +33,9 @@ class TailArgs(C.Structure):
     ]
 
 
+RDKV_K_ANY_ROWS = 65536   # flag on the decode entry points' k_row_bytes_max: K rows of any width and address
+
+
 class LayerView(C.Structure):
     """Mirror of ``rdkv_layer_view``; field order and types must match the header."""
     _fields_ = [

@@ -58,10 +58,9 @@ constexpr int KB_MAX = RDKV_KB_MAX;    // 16-channel blocks of the score product
 constexpr int DPAD_MAX = RDKV_DPAD_MAX;  // padded channel slots of a view (n_ch2_pad + n_ch4_pad + n_ch8)
 // dynamic shared memory behind the ring: folded queries in MMA fragment order, then the scratch the
 // fold reads (the group's query rows as fp32, the head's K scales, zero points and channel permutation)
-constexpr int QS_BYTES = KB_MAX * 32 * 8;
+// (those three only in launches without a prepared table)
 constexpr int FOLD_Q_BYTES = GH * 128 * 4;
 constexpr int FOLD_META_BYTES = 3 * DPAD_MAX * 2;
-constexpr int TAIL_BYTES = QS_BYTES + FOLD_Q_BYTES + FOLD_META_BYTES;
 constexpr float TWO24 = 16777216.f;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
@@ -295,10 +294,30 @@ __device__ __forceinline__ uint32_t lds32_unaligned(uint32_t a) {
   const uint32_t lo = lds32(a & ~3u), hi = lds32<4>(a & ~3u);
   return __funnelshift_r(lo, hi, (a & 3u) * 8);
 }
+// 32 bits from `shift` bits behind the word at `a` on (a: a whole word's address; two aligned loads).
+__device__ __forceinline__ uint32_t lds32_shifted(uint32_t a, uint32_t shift) {
+  return __funnelshift_r(lds32(a), lds32<4>(a), shift);
+}
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
   return v;
+}
+
+// Score products of one span of K codes: words of rows r (A) and r + 8 (B) of the group against the
+// folded queries.  The codes are masked in place into subnormal fp16 integers.
+// (2-bit codes: the span's two bytes in bytes 0 and 2 of the word)
+__device__ __forceinline__ void k_codes2_spread(float* sx, float* sy, uint32_t yA, uint32_t yB, uint2 p0, uint2 p1) {
+  mma16816(sx, yA & 0x00030003u, yB & 0x00030003u, yA & 0x000C000Cu, yB & 0x000C000Cu, p0.x, p0.y);
+  mma16816(sy, yA & 0x00300030u, yB & 0x00300030u, yA & 0x00C000C0u, yB & 0x00C000C0u, p1.x, p1.y);
+}
+__device__ __forceinline__ void k_codes4(float* sx, float* sy, uint32_t wA, uint32_t wB, uint2 p0, uint2 p1) {
+  const uint32_t vA = wA >> 8, vB = wB >> 8;
+  mma16816(sx, wA & 0x000F000Fu, wB & 0x000F000Fu, wA & 0x00F000F0u, wB & 0x00F000F0u, p0.x, p0.y);
+  mma16816(sy, vA & 0x000F000Fu, vB & 0x000F000Fu, vA & 0x00F000F0u, vB & 0x00F000F0u, p1.x, p1.y);
+}
+__device__ __forceinline__ void k_codes8(float* s, uint32_t wA, uint32_t wB, uint2 p0) {
+  mma16816(s, wA & 0x00FF00FFu, wB & 0x00FF00FFu, prmt(wA, 0u, 0x4341), prmt(wB, 0u, 0x4341), p0.x, p0.y);
 }
 
 // ── K channel-slot map: which padded channel slot feeds MMA k-index e of thread j ──
@@ -351,10 +370,11 @@ struct __align__(16) UnitRec {
   PhaseRec ph[4];
 };
 static_assert(sizeof(PhaseRec) == 64 && sizeof(UnitRec) == 304, "prepared-table records are read as int4 words");
-// One slot quadruple of the prepared K table: what thread `lane` of 16-channel block `kb` needs to
-// fold its four query elements — original channels, zero points (integers 0..255) and fp16 scales
-// (0 for a pad slot).  16 bytes; [unit][kb][lane].
+// One slot quadruple of the prepared K table: what the threads of place j = lane & 3 need of 16-channel
+// block `kb` to fold their four query elements — original channels, zero points (integers 0..255) and
+// fp16 scales (0 for a pad slot).  16 bytes; [unit][kb][j].
 struct __align__(16) KSlotRec { uint32_t perm4, zp4, sc01, sc23; };
+constexpr int KSLOT_RECS = 4;          // records per 16-channel block
 
 // Sequence parts: a head's rows are shared out phase by phase (every part gets its share of the
 // 2-bit, of the 4-bit, of the 8-bit and of the fp16 rows, so the parts read about the same bytes);
@@ -397,6 +417,7 @@ struct __align__(16) TileInfo {
 struct __align__(16) RangePlan { const unsigned char* src; int len; uint32_t dst_off; };
 struct __align__(16) TilePlan { RangePlan rg[6]; TileInfo info; };
 constexpr int PLAN_TILES = 32;         // tiles planned per round (one per staging lane)
+constexpr int PLAN_TILES_TAIL = 12;    // the same with an uncompressed tail (2.2 KB less: with K rows of up to 49 bytes there is room for three CTAs)
 
 template <int NPH>
 __device__ __forceinline__ TileDesc tile_of(const CtaGeom& G, int idx) {
@@ -599,6 +620,7 @@ struct EpiInfo {
 // of decode-appended tokens (a fifth tile phase of plain 16-bit K and V rows) and the token being
 // decoded, with the rotary embedding of the query rows and of the new key row applied on the way
 // in (TailArgs).  A separate instantiation: the other modes' code is not touched by it.
+constexpr uint32_t K_FEW = 64u;        // (k_spans in decode_state.inc) at most two spans per K segment
 constexpr int MODE_ATTN = 0, MODE_SCORES = 1, MODE_WEIGHTS = 2, MODE_ATTN_TAIL = 3;
 constexpr int TAIL_TILE = TILE_MAX / 8;             // tail rows per tile: K rows and V rows fill the V area together
 constexpr int TAILQ_BYTES = 8 * 32 * 8;             // the queries as fp16 B fragments of the tail's score product
@@ -607,7 +629,9 @@ static_assert(2 * TAIL_TILE * 256 <= V_STAGE, "a tail tile's K and V rows share 
 
 using TailArgs = rdkv_tail_args;
 
-template <int MODE>
+// WIDE: for views whose K rows may have any width (decode_tile_wide.inc); without it, rows of one span per
+// segment on whole words run the faster straight-line code and other rows a slow loop.
+template <int MODE, bool WIDE>
 #ifdef RDKV_MAXNREG
 __global__ void __maxnreg__(RDKV_MAXNREG)
 #else
@@ -623,6 +647,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
   constexpr bool TAIL = MODE == MODE_ATTN_TAIL;
   constexpr bool ATTN = MODE == MODE_ATTN || TAIL;
   constexpr int NPH = TAIL ? 5 : 4;                // tile phases
+  constexpr int PLAN = TAIL ? PLAN_TILES_TAIL : PLAN_TILES;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ rdkv_layer_view v;
   __shared__ CtaGeom G;
@@ -630,7 +655,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
   __shared__ float s_bias[FW][GH];                // zero-point bias of the folded queries: the warps' partial sums
   __shared__ EpiInfo s_epi;
   __shared__ TileInfo s_tile[FSTAGES];
-  __shared__ TilePlan s_plan[PLAN_TILES];          // private to the staging warp
+  __shared__ TilePlan s_plan[PLAN];          // private to the staging warp
   __shared__ __align__(8) uint64_t s_full[FSTAGES];   // tile in slot s has landed
 
   // Work items, one per CTA, in launch order: the first n_whole units (view, KV head, group of
@@ -657,7 +682,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
   // (a launch with a prepared table knows the largest number of K blocks of its views: the folded
   // queries take that many blocks of 256 bytes, not the 24 a view may have at most)
   const int qs_bytes = (nkb_max > 0 ? min(nkb_max, KB_MAX) : KB_MAX) * 256;
-  const int tail_bytes = qs_bytes + FOLD_Q_BYTES + FOLD_META_BYTES;
+  const int tail_bytes = qs_bytes + FOLD_Q_BYTES + (unit_recs != nullptr ? 0 : FOLD_META_BYTES);
   uint2* qsA = reinterpret_cast<uint2*>(tail);
   float* f_q = reinterpret_cast<float*>(tail + qs_bytes);                   // [gcnt][128] query rows as fp32
   uint16_t* f_sc = reinterpret_cast<uint16_t*>(tail + qs_bytes + FOLD_Q_BYTES);   // [d_pad] K scales (fp16 bits; launches without a prepared table)
@@ -770,9 +795,9 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
       for (int i = tid; i < (int)(sizeof(rdkv_layer_view) / 4); i += FW * 32) dst[i] = ldg_keep(src + i);
     }
     if (prepared && MODE != MODE_WEIGHTS) {
-      const int4* kp = reinterpret_cast<const int4*>(kslots + unit * nkb_max * 32 + lane);
-      if (warp < nkb_max) { const int4 t = ldg_keep4(kp + warp * 32); km0 = {(uint32_t)t.x, (uint32_t)t.y, (uint32_t)t.z, (uint32_t)t.w}; }
-      if (warp + FW < nkb_max) { const int4 t = ldg_keep4(kp + (warp + FW) * 32); km1 = {(uint32_t)t.x, (uint32_t)t.y, (uint32_t)t.z, (uint32_t)t.w}; }
+      const int4* kp = reinterpret_cast<const int4*>(kslots + unit * nkb_max * KSLOT_RECS + j);
+      if (warp < nkb_max) { const int4 t = ldg_keep4(kp + warp * KSLOT_RECS); km0 = {(uint32_t)t.x, (uint32_t)t.y, (uint32_t)t.z, (uint32_t)t.w}; }
+      if (warp + FW < nkb_max) { const int4 t = ldg_keep4(kp + (warp + FW) * KSLOT_RECS); km1 = {(uint32_t)t.x, (uint32_t)t.y, (uint32_t)t.z, (uint32_t)t.w}; }
     }
     if (MODE != MODE_WEIGHTS) {
       const int64_t q0 = ((int64_t)view_idx * H_q + hq0) * D;
@@ -1012,7 +1037,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
     for (int kb = warp; kb < kd.nkb; kb += FW, ++nb) {
       KSlotRec km = nb == 0 ? km0 : km1;
       if (nb >= 2) {
-        const int4 t = *(reinterpret_cast<const int4*>(kslots + unit * nkb_max * 32 + lane) + kb * 32);
+        const int4 t = *(reinterpret_cast<const int4*>(kslots + unit * nkb_max * KSLOT_RECS + j) + kb * KSLOT_RECS);
         km = {(uint32_t)t.x, (uint32_t)t.y, (uint32_t)t.z, (uint32_t)t.w};
       }
       float b = nb < 2 ? 0.f : bias_part;
@@ -1079,7 +1104,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
 
   if (warp == FW) {
     // ── staging warp ──────────────────────────────────────────────────────────
-    // Tiles are planned 32 at a time, one per lane (where each of a tile's six byte ranges
+    // Tiles are planned PLAN at a time, one per lane (where each of a tile's six byte ranges
     // starts, how long it is, where it goes), so that the per-tile work is a table look-up and
     // the copy instructions.  The warp only ever waits for a free slot; a tile's landing is
     // signalled to the compute warps by the copies themselves (mbarrier transaction bytes on
@@ -1091,10 +1116,10 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
     const uint64_t pol_stream = l2_policy_stream();
 #pragma unroll 1
     for (int it = 0; it < total_tiles; ++it) {
-      const int slot = it % PLAN_TILES;
-      if (slot == 0) {                                     // plan tiles [it, it + 32)
+      const int slot = it % PLAN;
+      if (slot == 0) {                                     // plan tiles [it, it + PLAN)
         __syncwarp();
-        if (it + lane < total_tiles) {
+        if ((PLAN == 32 || lane < PLAN) && it + lane < total_tiles) {
           const TileDesc t = tile_of<NPH>(G, it + lane);
           const int p = t.phase;
           TilePlan& P = s_plan[lane];
@@ -1260,7 +1285,11 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
     const int pb = (TAIL && p == 4) ? (warp + FW - ((t.phase >> 8) & (FW - 1))) % FW
                                     : (warp + FW - (it * (TILE_MAX / 128)) % FW) % FW;
 
+    if constexpr (WIDE) {
+#include "decode_tile_wide.inc"
+    } else {
 #include "decode_tile.inc"
+    }
     if (it + FSTAGES < total_tiles) bar_arrive(BAR_FREE + stage, CTA_THREADS);   // slot may be refilled
   }
 
@@ -1319,7 +1348,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
 //     to run dry puts the counters (work[0], work[1]) back to zero for the next launch.
 struct ItemInfo { int n2p, n4p, n8c, total, item, pad0, pad1, pad2; };
 
-template <int MODE>
+template <int MODE, bool WIDE>
 __global__ void __launch_bounds__(CTA_THREADS, RDKV_MINB)
 decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, int chunk_rows, int k_chunks,
                       int n_whole, int n_items, int stage_bytes, float* __restrict__ partials,
@@ -1347,7 +1376,7 @@ decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, i
   uint2* qsA = reinterpret_cast<uint2*>(tail);
   const int q_elt = q_dtype == RDKV_F32 ? 4 : 2;
   const int hdr_q_bytes = GH * D * q_elt;                  // raw query rows of an item
-  const int hdr_bytes = hdr_q_bytes + nkb_max * 32 * (int)sizeof(KSlotRec);
+  const int hdr_bytes = hdr_q_bytes + nkb_max * KSLOT_RECS * (int)sizeof(KSlotRec);
   unsigned char* hdr0 = tail + nkb_max * 256;
   constexpr int BAR_COMPUTE = 1 + FSTAGES;
   const struct { const float* mask; int64_t mask_row_stride; } v = {nullptr, 0};   // (no mask in this form)
@@ -1480,8 +1509,8 @@ decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, i
         const int uy = ni < n_whole ? ni : n_whole + (ni - n_whole) / k_chunks;
         const int64_t nu = (int64_t)(uy / hy) * (H_q / g) + (uy % hy) / n_hgrp;
         if (lane < 3) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const unsigned char*>(unit_recs + nu) + 128 * lane));
-        else if (lane - 3 < (nkb_max * 32 * (int)sizeof(KSlotRec) + 127) / 128)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const unsigned char*>(kslots + nu * nkb_max * 32) + 128 * (lane - 3)));
+        else if (lane - 3 < (nkb_max * KSLOT_RECS * (int)sizeof(KSlotRec) + 127) / 128)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const unsigned char*>(kslots + nu * nkb_max * KSLOT_RECS) + 128 * (lane - 3)));
       }
 #endif
 #pragma unroll 1
@@ -1538,8 +1567,8 @@ decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, i
           rp.len = gcnt * D * q_elt; dst = smem_u32(hdr);
         }
         if (it == 0 && lane == 7) {
-          rp.src = reinterpret_cast<const unsigned char*>(kslots + unit * nkb_max * 32);
-          rp.len = nkb_max * 32 * (int)sizeof(KSlotRec); dst = smem_u32(hdr + hdr_q_bytes);
+          rp.src = reinterpret_cast<const unsigned char*>(kslots + unit * nkb_max * KSLOT_RECS);
+          rp.len = nkb_max * KSLOT_RECS * (int)sizeof(KSlotRec); dst = smem_u32(hdr + hdr_q_bytes);
         }
         const bool v_tma = (ti.phase >> 16) & 1, v_lanes = (ti.phase >> 17) & 1;   // how the V rows travel
         const uintptr_t a = reinterpret_cast<uintptr_t>(rp.src), al = a & ~(uintptr_t)15;
@@ -1646,7 +1675,7 @@ decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, i
 #pragma unroll 1
         for (int kb = warp; kb < kd.nkb; kb += FW, ++nb) {
           float b = nb < 2 ? 0.f : bias_part;
-          fold_block(hk[kb * 32 + lane], kb, b);
+          fold_block(hk[kb * KSLOT_RECS + j], kb, b);
           bias_part = nb < 2 ? bias_part + b : b;
         }
         bias_part += __shfl_xor_sync(0xffffffffu, bias_part, 1);
@@ -1682,7 +1711,11 @@ decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, i
         const int p = t.phase & 3;
         const int nblocks = (t.n + 31) >> 5;
         const int pb = (warp + FW - (it * (TILE_MAX / 128)) % FW) % FW;
+        if constexpr (WIDE) {
+#include "decode_tile_wide.inc"
+        } else {
 #include "decode_tile.inc"
+        }
         if (it + 1 < n_it) {                               // (the item's last slot is handed back after the merge)
           __syncwarp();
           if (lane == 0) mbar_arrive(&s_empty[stage]);
@@ -1750,8 +1783,8 @@ decode_prepare_kernel(const rdkv_layer_view* __restrict__ views, int H_kv, int n
   const uint16_t* sc = v.k_scale + (int64_t)h * d_pad;
   const uint16_t* zp = v.k_zp + (int64_t)h * d_pad;
   const int64_t* perm = v.k_perm + (int64_t)h * v.k_perm_head_stride;
-  for (int i = threadIdx.x; i < nkb_max * 32; i += blockDim.x) {
-    const int kb = i >> 5, j = i & 3;
+  for (int i = threadIdx.x; i < nkb_max * KSLOT_RECS; i += blockDim.x) {
+    const int kb = i / KSLOT_RECS, j = i % KSLOT_RECS;
     KSlotRec rec = {0u, 0u, 0u, 0u};
     if (kb < kd.nkb) {
 #pragma unroll
@@ -1766,10 +1799,11 @@ decode_prepare_kernel(const rdkv_layer_view* __restrict__ views, int H_kv, int n
         if (e < 2) rec.sc01 |= (uint32_t)sc[slot] << (16 * e); else rec.sc23 |= (uint32_t)sc[slot] << (16 * (e - 2));
       }
     }
-    kslots[unit * nkb_max * 32 + i] = rec;
+    kslots[unit * nkb_max * KSLOT_RECS + i] = rec;
   }
   if (threadIdx.x == 0) {
     const HeadCounts hc = head_counts(v, h);
+    bool simple = kd.nsp2 == 1 && kd.nsp4 == 1 && kd.nkb8 == 1 && !(kd.sub2 & 1) && !(kd.sub4 & 3) && !(kd.n8 & 3);   // the straight-line code takes its K rows
     bool fast = true, mapped = true;                      // mapped: the V rows of every spaced-out phase can come through a tensor map
     UnitRec u;
     for (int p = 0; p < 4; ++p) {                          // the whole head, phase by phase (as the kernel's geometry does per chunk)
@@ -1792,6 +1826,7 @@ decode_prepare_kernel(const rdkv_layer_view* __restrict__ views, int H_kv, int n
         if (kd.sub2) fast = fast && blocks_inside(a2, a2 + (int64_t)n * kd.sub2, v.k2, v.k2 + v.k2_bytes);
         if (kd.sub4) fast = fast && blocks_inside(a4, a4 + (int64_t)n * kd.sub4, v.k4, v.k4 + v.k4_bytes);
         if (kd.n8) fast = fast && blocks_inside(a8, a8 + (int64_t)n * kd.n8, v.k8, v.k8 + v.k8_bytes);
+        simple = simple && ((reinterpret_cast<uintptr_t>(a2) & 1) | (reinterpret_cast<uintptr_t>(a4) & 3) | (reinterpret_cast<uintptr_t>(a8) & 3)) == 0;
         fast = fast && vb != nullptr && blocks_inside(vb, vb + (int64_t)n * phase_row_bytes(p), vlo, vlo + vext);
         if (p < 3) {
           fast = fast && gsc != nullptr && gzp != nullptr;
@@ -1812,7 +1847,7 @@ decode_prepare_kernel(const rdkv_layer_view* __restrict__ views, int H_kv, int n
       u.ph[p].k2 = a2; u.ph[p].k4 = a4; u.ph[p].k8 = a8; u.ph[p].vrow = vb; u.ph[p].sc = gsc; u.ph[p].zp = gzp;
     }
     u.n2 = hc.n2; u.n4 = hc.n4; u.n8 = hc.n8; u.n16 = hc.n16;
-    u.flags = (fast ? 1 : 0) | (fast && mapped ? 2 : 0); u.nkb = kd.nkb; u.n_ch2_pad = kd.n2p; u.n_ch4_pad = kd.n4p;
+    u.flags = (fast ? 1 : 0) | (fast && mapped ? 2 : 0) | (simple ? 4 : 0); u.nkb = kd.nkb; u.n_ch2_pad = kd.n2p; u.n_ch4_pad = kd.n4p;
     u.n_ch8 = kd.n8; u.max_t_v = v.max_t_v;
     const uintptr_t vm = v_maps != nullptr ? reinterpret_cast<uintptr_t>(v_maps + (unit / H_kv) * 4 * 128) : 0;
     u.vmaps_lo = (unsigned)(vm & 0xFFFFFFFFu); u.vmaps_hi = (unsigned)(vm >> 32);
@@ -1831,6 +1866,9 @@ static int launch_fused(const rdkv_layer_view* views, int n_views, const void* q
   const int g = H_q / H_kv;
   const int n_hgrp = (g + GH - 1) / GH;
   const int64_t units = (int64_t)n_views * H_kv * n_hgrp;
+  const bool wide = MODE != MODE_WEIGHTS && (k_row_bytes_max & RDKV_K_ANY_ROWS) != 0;
+  k_row_bytes_max &= ~RDKV_K_ANY_ROWS;
+  const auto kernel = wide ? decode_fused_kernel<MODE, MODE != MODE_WEIGHTS> : decode_fused_kernel<MODE, false>;
   if (n_whole < 0 || n_whole > units) return RDKV_ERR_BAD_ARG;
   const int64_t items = n_whole + (units - n_whole) * n_chunks;
   if (items > 0x7fffffffLL) return RDKV_ERR_TOO_LARGE;
@@ -1840,7 +1878,7 @@ static int launch_fused(const rdkv_layer_view* views, int n_views, const void* q
     return RDKV_ERR_BAD_ARG;
   const int stage_bytes = align128i(stage_capacity(k_row_bytes_max));   // (a tile's V box lands on a 128-byte boundary)
   const int qs_bytes = (nkb_max > 0 ? std::min(nkb_max, KB_MAX) : KB_MAX) * 256;   // (as the kernel lays it out)
-  size_t smem = (size_t)FSTAGES * stage_bytes + qs_bytes + FOLD_Q_BYTES + FOLD_META_BYTES +
+  size_t smem = (size_t)FSTAGES * stage_bytes + qs_bytes + FOLD_Q_BYTES + (unit_recs != nullptr ? 0 : FOLD_META_BYTES) +
                 (MODE == MODE_ATTN_TAIL ? TAIL_EXTRA_BYTES : 0);
   const size_t epilogue = (size_t)FW * GH * D * sizeof(float);
   if (smem < epilogue) smem = epilogue;
@@ -1848,9 +1886,9 @@ static int launch_fused(const rdkv_layer_view* views, int n_views, const void* q
   TailArgs ta;
   memset(&ta, 0, sizeof(ta));
   if (tail != nullptr) ta = *tail;
-  cudaError_t e = cudaFuncSetAttribute(decode_fused_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
-  decode_fused_kernel<MODE><<<(unsigned)items, CTA_THREADS, smem, (cudaStream_t)stream>>>(
+  kernel<<<(unsigned)items, CTA_THREADS, smem, (cudaStream_t)stream>>>(
       views, q, q_dtype, H_q, g, chunk_rows, n_chunks, n_whole, stage_bytes, partials, out, status, aux, aux_stride, t_eff,
       reinterpret_cast<const UnitRec*>(unit_recs), reinterpret_cast<const KSlotRec*>(kslots), nkb_max, unit_ctr, merged,
       row_begin, row_end, part, parts, ta);
@@ -1862,6 +1900,7 @@ static int check_fused_args(const rdkv_layer_view* views, int n_views, const voi
   if (views == nullptr || q == nullptr || n_views < 0) return RDKV_ERR_BAD_ARG;
   if (q_dtype < RDKV_F16 || q_dtype > RDKV_F32) return RDKV_ERR_BAD_ARG;
   if (H_q <= 0 || H_kv <= 0 || H_q % H_kv != 0) return RDKV_ERR_BAD_SHAPE;
+  k_row_bytes_max &= ~RDKV_K_ANY_ROWS;
   if (k_row_bytes_max <= 0 || k_row_bytes_max > 224) return RDKV_ERR_BAD_SHAPE;
   return RDKV_OK;
 }
@@ -1883,7 +1922,7 @@ extern "C" int rdkv_decode_k_blocks(int n_ch2_pad, int n_ch4_pad, int n_ch8) {
 
 extern "C" int64_t rdkv_decode_prepared_bytes(int64_t n_units, int nkb_max, int which) {
   if (n_units < 0 || nkb_max < 0) return -1;
-  return which == 0 ? n_units * (int64_t)sizeof(UnitRec) : n_units * nkb_max * 32 * (int64_t)sizeof(KSlotRec);
+  return which == 0 ? n_units * (int64_t)sizeof(UnitRec) : n_units * nkb_max * KSLOT_RECS * (int64_t)sizeof(KSlotRec);
 }
 
 // The driver's tensor-map encoder, found through the runtime (the library does not link the driver).
@@ -2085,25 +2124,27 @@ extern "C" int rdkv_decode_attn_persistent(const rdkv_layer_view* views, int n_v
   if (n_whole_units < 0 || n_whole_units > units) return RDKV_ERR_BAD_ARG;
   const int64_t items = n_whole_units + (units - n_whole_units) * n_chunks;
   if (items > 0x7fffffffLL) return RDKV_ERR_TOO_LARGE;
+  const auto kernel = (k_row_bytes_max & RDKV_K_ANY_ROWS) ? decode_persist_kernel<MODE_ATTN, true> : decode_persist_kernel<MODE_ATTN, false>;
+  k_row_bytes_max &= ~RDKV_K_ANY_ROWS;
   const int stage_bytes = align128i(stage_capacity(k_row_bytes_max));   // (a tile's V box lands on a 128-byte boundary)
   const int q_elt = q_dtype == RDKV_F32 ? 4 : 2;
   size_t smem = (size_t)FSTAGES * stage_bytes + (size_t)nkb_max * 256 +
-                2 * ((size_t)GH * D * q_elt + (size_t)nkb_max * 32 * sizeof(KSlotRec));
+                2 * ((size_t)GH * D * q_elt + (size_t)nkb_max * KSLOT_RECS * sizeof(KSlotRec));
   const size_t epilogue = (size_t)FW * GH * D * sizeof(float);
   if ((size_t)stage_bytes < epilogue) return RDKV_ERR_BAD_SHAPE;     // the merge works inside one ring slot
   if (smem > 227 * 1024) return RDKV_ERR_TOO_LARGE;
-  cudaError_t e = cudaFuncSetAttribute(decode_persist_kernel<MODE_ATTN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_persist_kernel<MODE_ATTN>, CTA_THREADS, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, CTA_THREADS, smem) != cudaSuccess ||
       per_sm <= 0) {
     g_last_cuda_error = (int)cudaGetLastError();
     return RDKV_ERR_LAUNCH;
   }
   const int64_t slots = (int64_t)sms * per_sm;
   const unsigned grid = (unsigned)(items < slots ? items : slots);
-  decode_persist_kernel<MODE_ATTN><<<grid, CTA_THREADS, smem, (cudaStream_t)stream>>>(
+  kernel<<<grid, CTA_THREADS, smem, (cudaStream_t)stream>>>(
       q, q_dtype, H_q, g, chunk_rows, n_chunks, n_whole_units, (int)items, stage_bytes, partials, out, status,
       reinterpret_cast<const UnitRec*>(unit_recs), reinterpret_cast<const KSlotRec*>(k_slots), nkb_max, unit_counters,
       out_record, row_begin, row_end, seq_part, seq_parts, work_counters);

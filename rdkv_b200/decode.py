@@ -16,7 +16,7 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 from torch import Tensor
 
-from ._lib import (HEAD_DIM, PARTIAL_STRIDE, LayerView, TailArgs, check, lib, ptr, q_dtype_tag, require_cuda,
+from ._lib import (HEAD_DIM, PARTIAL_STRIDE, RDKV_K_ANY_ROWS, LayerView, TailArgs, check, lib, ptr, q_dtype_tag, require_cuda,
                    stream_ptr)
 from .packing import PackedKVLayer, layer_identity, layer_view
 
@@ -97,6 +97,7 @@ class DecodeTable:
         n_units = self.n_views * self.H_kv
         self._unit_rec_bytes = int(L.rdkv_decode_prepared_bytes(1, self.nkb_max, 0))
         self.unit_recs = torch.empty(L.rdkv_decode_prepared_bytes(n_units, self.nkb_max, 0), dtype=torch.uint8, device=self.device)
+        self._k_slot_bytes = int(L.rdkv_decode_prepared_bytes(1, self.nkb_max, 1))
         self.k_slots = torch.empty(L.rdkv_decode_prepared_bytes(n_units, self.nkb_max, 1), dtype=torch.uint8, device=self.device)
         self.unit_ctr = torch.zeros(self.n_views * self.H_kv * n_hgrp, dtype=torch.int32, device=self.device)
         # item counters of the persistent form: a pair per launch that may be in flight at the same time
@@ -111,9 +112,17 @@ class DecodeTable:
         # (flag bit 0 of its prepared record; read back once, here)
         self.persistent = None if persistent is None else bool(persistent)
         self._all_fast = False
+        # whether K rows need the kernel for rows of any width: by their channel counts here, by the
+        # prepared records (which know the rows' addresses too) where there are some
+        self._wide = any(n2 // 4 > 8 or n4 // 2 > 16 or n8 > 16 or n2 // 4 % 2 or n4 // 2 % 4 or n8 % 4 or not (n2 and n4 and n8)
+                         for n2, n4, n8 in ((int(vw.n_ch2_pad), int(vw.n_ch4_pad), int(vw.n_ch8)) for vw in views))
         if not self.live_counts:
             recs = self.unit_recs.view(torch.int32).view(n_units, self._unit_rec_bytes // 4)
-            self._all_fast = bool(((recs[:, 4] & 3) == 3).all().item())   # (bit 1: the V rows come through tensor maps)
+            # (bit 1: the V rows come through tensor maps; bit 2: K rows of one span per segment on whole words)
+            flags = recs[:, 4]
+            self._all_fast, simple = torch.stack([((flags & 3) == 3).all(), ((flags & 4) != 0).all()]).tolist()
+            self._wide = not simple
+        self.k_rows_arg = self.k_row_bytes_max | (RDKV_K_ANY_ROWS if self._wide else 0)
 
     CTAS_PER_SM = 3                      # resident CTAs of the fused kernel per SM
     WORK_CTR_SLOTS = 64                  # launches of one table that may overlap (view ranges on streams of their own)
@@ -260,7 +269,7 @@ def _launch_fused(q: Tensor, table: DecodeTable, partials: Optional[Tensor], out
         n_chunks, chunk_rows = table.plan(v1 - v0)[:2]
     check(lib().rdkv_decode_attn_partial(table.views.data_ptr() + v0 * C.sizeof(LayerView), v1 - v0,
                                          off(q, HEAD_DIM), q_dtype_tag(q), table.H_q,
-                                         table.H_kv, chunk_rows, n_chunks, table.k_row_bytes_max,
+                                         table.H_kv, chunk_rows, n_chunks, table.k_rows_arg,
                                          off(partials, n_chunks * PARTIAL_STRIDE), off(out, HEAD_DIM),
                                          ptr(table.status), stream_ptr(q.device)),
           "rdkv_decode_attn_partial")
@@ -335,9 +344,9 @@ def _launch_units(q: Tensor, table: DecodeTable, out: Optional[Tensor], v0: int 
     with torch.cuda.device(table.device):
         check(fn(table.views.data_ptr() + v0 * C.sizeof(LayerView), v1 - v0,
                                      off(q, HEAD_DIM), q_dtype_tag(q), table.H_q, table.H_kv, rows_k, k, n_whole, r0, r1, sp_i, sp_n,
-                                     table.k_row_bytes_max,
+                                     table.k_rows_arg,
                                      None if table.live_counts else table.unit_recs.data_ptr() + v0 * table.H_kv * table._unit_rec_bytes,
-                                     None if table.live_counts else table.k_slots.data_ptr() + v0 * table.H_kv * table.nkb_max * 512,
+                                     None if table.live_counts else table.k_slots.data_ptr() + v0 * table.H_kv * table._k_slot_bytes,
                                      0 if table.live_counts else table.nkb_max,
                                      off(ws, k * PARTIAL_STRIDE), table.unit_ctr.data_ptr() + v0 * hy * 4, *extra,
                                      off(out, HEAD_DIM), off(out_record, PARTIAL_STRIDE),

@@ -53,7 +53,7 @@ def k_mixed_qk_dot_into(Q: torch.Tensor, packed_layer, T_eff: int, out: torch.Te
             Q = Q.contiguous()
         rows = 256
         check(lib().rdkv_decode_scores(ptr(table.views), 1, ptr(Q), q_dtype_tag(Q), H_q, table.H_kv, rows,
-                                       -(-int(T_eff) // rows), table.k_row_bytes_max, int(T_eff), ptr(out),
+                                       -(-int(T_eff) // rows), table.k_rows_arg, int(T_eff), ptr(out),
                                        out.stride(0), ptr(table.status), stream_ptr(Q.device)), "rdkv_decode_scores")
         return
     if Q.stride(1) != 1:

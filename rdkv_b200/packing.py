@@ -108,6 +108,17 @@ def _as_fp16_rows(x: Tensor, name: str) -> Tensor:
     return x
 
 
+def _empty_padded(shape: Sequence[int], dtype: torch.dtype, device) -> Tensor:
+    """Uninitialised tensor whose storage goes on for at least 16 bytes behind its last element.  The decode
+    kernel copies the 16-byte blocks that cover a range of rows: without the slack the last head's
+    blocks would stick out of a tensor whose length is no multiple of 16 bytes (odd channel counts,
+    odd row counts), and the launch would have to take slower, guarded copies."""
+    n = 1
+    for x in shape:
+        n *= int(x)
+    return torch.empty(n + 16, dtype=dtype, device=device)[:n].view(*shape)
+
+
 # ── C-ABI wrappers ───────────────────────────────────────────────────────────
 
 def partition_by_bits(bits: Tensor, mode: int, fill: bool = True) -> Tuple[Tensor, Tensor]:
@@ -147,8 +158,8 @@ def _launch_pack_v(V: Tensor, order: Optional[Tensor], order_rs: int, counts: Op
     v4 = torch.empty((1, H, m4, D // 2), **u8) if m4 else None
     v8 = torch.empty((1, H, m8, D), **u8) if m8 else None
     v16 = torch.empty((1, H, m16, D), dtype=torch.float16, device=dev) if m16 else None
-    scale = torch.empty((1, H, max_t_v, 1), dtype=torch.float16, device=dev)
-    zp = torch.empty_like(scale)
+    scale = _empty_padded((1, H, max_t_v, 1), torch.float16, dev)
+    zp = _empty_padded((1, H, max_t_v, 1), torch.float16, dev)
     check(lib().rdkv_pack_v(ptr(V), V.stride(1), V.stride(2), H, D, ptr(order), order_rs, ptr(counts),
                             counts_rs, n_identity, identity_bits, m2, m4, m8, m16, ptr(v2), ptr(v4), ptr(v8),
                             ptr(v16), ptr(scale), ptr(zp), max_t_v, override, stream_ptr(dev)),
@@ -167,15 +178,14 @@ def _launch_pack_k(K: Tensor, tok_order, tok_order_rs, tok_counts, tok_counts_rs
     _, H, _, D = K.shape
     dev = K.device
     d_pad = n2p + n4p + n8p
-    u8 = dict(dtype=torch.uint8, device=dev)
     i64 = dict(dtype=torch.int64, device=dev)
     if override:
         k2 = k4 = None
-        k8 = torch.empty((1, H, t_k, d_pad), **u8)
+        k8 = torch.empty((1, H, t_k, d_pad), dtype=torch.uint8, device=dev)
     else:
-        k2 = torch.empty((1, H, t_k, n2p // 4), **u8) if n2p else None
-        k4 = torch.empty((1, H, t_k, n4p // 2), **u8) if n4p else None
-        k8 = torch.empty((1, H, t_k, n8p), **u8) if n8p else None
+        k2 = _empty_padded((1, H, t_k, n2p // 4), torch.uint8, dev) if n2p else None
+        k4 = _empty_padded((1, H, t_k, n4p // 2), torch.uint8, dev) if n4p else None
+        k8 = _empty_padded((1, H, t_k, n8p), torch.uint8, dev) if n8p else None
     scale = torch.empty((1, H, 1, d_pad), dtype=torch.float16, device=dev)
     zp = torch.empty_like(scale)
     sort_idx = torch.empty((H, d_kept_max), **i64)
@@ -545,11 +555,11 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
     V4 = torch.empty((L, H, R4, D // 2), **u8) if R4 else None
     V8 = torch.empty((L, H, R8, D), **u8) if R8 else None
     V16 = torch.empty((L, H, R16, D), **f16) if R16 else None
-    VS = torch.empty((L, H, max(RM, 1), 1), **f16)
-    VZ = torch.empty_like(VS)
-    K2 = torch.empty((L, H, RK, N2P // 4), **u8) if N2P else None
-    K4 = torch.empty((L, H, RK, N4P // 2), **u8) if N4P else None
-    K8 = torch.empty((L, H, RK, N8P), **u8) if N8P else None
+    VS = _empty_padded((L, H, max(RM, 1), 1), torch.float16, dev)
+    VZ = _empty_padded((L, H, max(RM, 1), 1), torch.float16, dev)
+    K2 = _empty_padded((L, H, RK, N2P // 4), torch.uint8, dev) if N2P else None
+    K4 = _empty_padded((L, H, RK, N4P // 2), torch.uint8, dev) if N4P else None
+    K8 = _empty_padded((L, H, RK, N8P), torch.uint8, dev) if N8P else None
     KS = torch.empty((L, H, 1, d_pad), **f16)
     KZ = torch.empty_like(KS)
     SORT = torch.empty((L, H, DK), **i64)
@@ -888,7 +898,11 @@ def layer_view(pl: PackedKVLayer, V16: Optional[Tensor] = None, n_v16_per_head: 
     v = LayerView()
     keep = []
 
-    def put(name, t, stride_name=None, stride_dim=0, bytes_=False, extent_name=None):
+    def room(t):
+        # bytes from the base pointer to the end of the tensor's storage: what may be read at all
+        return t.untyped_storage().nbytes() - t.storage_offset() * t.element_size()
+
+    def put(name, t, stride_name=None, stride_dim=0, bytes_=False, extent_name=None, whole_storage=False):
         t = _squeeze_h(t)
         if t is None or t.numel() == 0:
             setattr(v, name, None)
@@ -903,16 +917,17 @@ def layer_view(pl: PackedKVLayer, V16: Optional[Tensor] = None, n_v16_per_head: 
         if stride_name:
             setattr(v, stride_name, t.stride(stride_dim) * (t.element_size() if bytes_ else 1))
         if extent_name:
-            # last addressable byte + 1, relative to the base pointer
+            # last addressable byte + 1, relative to the base pointer (rows that are copied block by block:
+            # up to the end of the storage)
             last = sum((n - 1) * st for n, st in zip(t.shape, t.stride()))
-            setattr(v, extent_name, (last + 1) * t.element_size())
+            setattr(v, extent_name, room(t) if whole_storage else (last + 1) * t.element_size())
         return t
 
     n2c, n4c, n8c = (int(x) for x in pl.K_ch_seg_bounds)
     v.n_ch2_pad, v.n_ch4_pad, v.n_ch8 = _pad_to(n2c, 4), _pad_to(n4c, 2), n8c
-    put("k2", pl.K_2bit if v.n_ch2_pad else None, "k2_head_stride", 0, True, "k2_bytes")
-    put("k4", pl.K_4bit if v.n_ch4_pad else None, "k4_head_stride", 0, True, "k4_bytes")
-    put("k8", pl.K_8bit if v.n_ch8 else None, "k8_head_stride", 0, True, "k8_bytes")
+    put("k2", pl.K_2bit if v.n_ch2_pad else None, "k2_head_stride", 0, True, "k2_bytes", True)
+    put("k4", pl.K_4bit if v.n_ch4_pad else None, "k4_head_stride", 0, True, "k4_bytes", True)
+    put("k8", pl.K_8bit if v.n_ch8 else None, "k8_head_stride", 0, True, "k8_bytes", True)
     sc = _squeeze_h(pl.K_ch_scale)
     put("k_scale", sc.reshape(sc.shape[0], -1) if sc is not None and sc.numel() else None)
     zp = _squeeze_h(pl.K_ch_zp)
@@ -934,8 +949,10 @@ def layer_view(pl: PackedKVLayer, V16: Optional[Tensor] = None, n_v16_per_head: 
     vs = _squeeze_h(pl.V_scale)
     vz = _squeeze_h(pl.V_zp)
     put("v_scale", vs.reshape(vs.shape[0], -1) if vs.numel() else None, "v_meta_head_stride", 0, False,
-        "v_meta_bytes")
-    put("v_zp", vz.reshape(vz.shape[0], -1) if vz.numel() else None)
+        "v_meta_bytes", True)
+    zt = put("v_zp", vz.reshape(vz.shape[0], -1) if vz.numel() else None)
+    if zt is not None and v.v_scale:
+        v.v_meta_bytes = min(v.v_meta_bytes, room(zt))
     if pl.seg_bounds_per_head is not None:
         sb = pl.seg_bounds_per_head
         if sb.dtype != torch.int32 or not sb.is_contiguous():

@@ -1,0 +1,49 @@
+"""Decode over layers whose K rows have any number of bytes at any address: every way the fused kernel
+reads K codes (one span of whole words, two spans and many spans at any byte), odd row counts that
+put V scales on odd half-words, and heads of very different lengths, against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import assert_attn_close, layer_to_np, to_np
+
+pytestmark = pytest.mark.gpu
+
+# channels per head of 8, 4 and 2 bits: aligned single spans, odd widths, empty segments, two spans at the
+# limit, more than two spans
+CHANNELS = [(16, 24, 24), (24, 31, 27), (23, 31, 35), (5, 32, 0), (0, 3, 61), (32, 64, 32), (1, 0, 0), (33, 40, 50), (3, 17, 100)]
+
+
+def _layer(counts, T, kept, seed, g, H=2):
+    from rdkv_b200 import synth
+    from rdkv_b200.packing import pack_kv
+    K, V = synth.make_kv(H, T, seed=seed)
+    vb = synth.make_v_bits(H, T, max(kept), seed=seed, per_head_N=kept)
+    kb = synth.make_k_bits(H, seed=seed, mix=tuple(zip((8, 4, 2), counts)))
+    if sum(counts) > 4:                                      # another count in the second head: padded slots
+        kb[1, torch.nonzero(kb[1] == (8 if counts[0] else 4))[0]] = 0
+    return pack_kv(K.cuda(), V.cuda(), vb.cuda(), kb.cuda(), g)
+
+
+@pytest.mark.parametrize("counts", CHANNELS)
+@pytest.mark.parametrize("kept", [(301, 77), (1, 640)])
+def test_k_rows_of_any_width(counts, kept):
+    from oracle import ref_attention as RA
+    from rdkv_b200 import synth
+    from rdkv_b200.decode import DecodeTable, packed_decode_attention
+    g, H = 4, 2
+    layers = [_layer(counts, 700, list(kept), 11, g), _layer(counts, 701, list(kept)[::-1], 12, g)]
+    q = synth.make_q(H * g, seed=5, batch=2)
+    wants = [RA.decode_attention(q[i].numpy(), layer_to_np(pl), to_np(nv))[0] for i, (pl, nv) in enumerate(layers)]
+    for persistent in (False, True):
+        table = DecodeTable([p for p, _ in layers], [n for _, n in layers], H * g, persistent=persistent)
+        assert table._all_fast, "the packed rows lie in copyable 16-byte blocks"
+        out = packed_decode_attention(q.cuda(), table)
+        table.check_status()
+        for i, want in enumerate(wants):
+            assert_attn_close(to_np(out[i]), want, f"view {i}, persistent {persistent}")
+    # without a snapshot (counts and scales read by every CTA) and through the two separate operators
+    live = DecodeTable([p for p, _ in layers], [n for _, n in layers], H * g, live_counts=True)
+    out = packed_decode_attention(q.cuda(), live)
+    for i, want in enumerate(wants):
+        assert_attn_close(to_np(out[i]), want, f"live view {i}")
