@@ -455,6 +455,22 @@ int rdkv_unpack_layer(const rdkv_layer_view* view, int H_kv, int D, const int64_
                       int n_ch8, uint16_t* k_out, uint16_t* v_out, int64_t out_head_stride, int rows_out,
                       void* stream);
 
+/* The same for several layers at once (one launch per 16 layers).  `jobs` is a HOST array, copied into the
+ * launches; the fields are rdkv_unpack_layer's arguments. */
+typedef struct rdkv_unpack_job {
+  rdkv_layer_view view;
+  const int64_t* k_sort_idx;
+  int64_t k_sort_idx_head_stride;
+  const int32_t* k_ch_counts;
+  int32_t n_ch2, n_ch4, n_ch8, H_kv;
+  uint16_t* k_out;
+  uint16_t* v_out;
+  int64_t out_head_stride;
+  int32_t rows_out, reserved;
+} rdkv_unpack_job;
+int rdkv_sizeof_unpack_job(void);
+int rdkv_unpack_layers(const rdkv_unpack_job* jobs, int n_jobs, int D, void* stream);
+
 /* ── prefill: every layer of a cache in one pass ──────────────────────────────
  * The reference packs a whole cache layer by layer (build_packed_cache,
  * obkv_accel/packing.py:1323-1421; driver loop obkv_fast.py:1098-1166); here the

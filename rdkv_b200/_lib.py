@@ -84,6 +84,16 @@ class PackJob(C.Structure):
 
 _lib: Optional[C.CDLL] = None
 
+class UnpackJob(C.Structure):
+    """Mirror of ``rdkv_unpack_job`` (one layer of a batched unpack); field order and types must match the header."""
+    _fields_ = [
+        ("view", LayerView), ("k_sort_idx", C.c_void_p), ("k_sort_idx_head_stride", C.c_int64), ("k_ch_counts", C.c_void_p),
+        ("n_ch2", C.c_int32), ("n_ch4", C.c_int32), ("n_ch8", C.c_int32), ("H_kv", C.c_int32),
+        ("k_out", C.c_void_p), ("v_out", C.c_void_p), ("out_head_stride", C.c_int64),
+        ("rows_out", C.c_int32), ("reserved", C.c_int32),
+    ]
+
+
 _i, _i64, _p, _f = C.c_int, C.c_int64, C.c_void_p, C.c_float
 
 _PROTOTYPES = {
@@ -123,6 +133,8 @@ _PROTOTYPES = {
     "rdkv_score_pool": ([_p, _i64, _i, _i, _i, _i, _i, _p, _i64, _i, _p], _i),
     "rdkv_block_scores": ([_p, _i, _i64, _i64, _p, _i, _i64, _i64, _i, _i, _i, _i, _i, _i, _p, _p, _p], _i),
     "rdkv_unpack_layer": ([_p, _i, _i, _p, _i64, _p, _i, _i, _i, _p, _p, _i64, _i, _p], _i),
+    "rdkv_sizeof_unpack_job": ([], _i),
+    "rdkv_unpack_layers": ([_p, _i, _i, _p], _i),
     "rdkv_sizeof_pack_job": ([], _i),
     "rdkv_pack_kv_batched": ([_p, _i, _i, _i, _i, _i, _i, _i, _i, _p], _i),
     "rdkv_knapsack_batched": ([_p, _i64, _i, _i, _p, C.POINTER(_f), C.POINTER(_f), _i, _i, _f, _p, _p, _p], _i),
@@ -155,6 +167,8 @@ def lib() -> C.CDLL:
             raise RuntimeError("rdkv_b200: rdkv_tail_args layout mismatch between header and binding")
         if handle.rdkv_sizeof_pack_job() != C.sizeof(PackJob):
             raise RuntimeError("rdkv_b200: rdkv_pack_job layout mismatch between header and binding")
+        if handle.rdkv_sizeof_unpack_job() != C.sizeof(UnpackJob):
+            raise RuntimeError("rdkv_b200: rdkv_unpack_job layout mismatch between header and binding")
         _lib = handle
     return _lib
 

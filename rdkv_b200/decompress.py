@@ -3,7 +3,8 @@
 Mirrors ``unpack_k_mixed`` (obkv_accel/packing.py:581-709), ``unpack_v_segment``
 (:1427-1444) and ``unpack_trizone_to_past_kv`` with its helpers
 (obkv_accel/trizone_decompress.py:43-333): same names, arguments and results, computed
-by one CUDA launch per layer (``rdkv_unpack_layer``).  Tensors must be on a CUDA device.
+by one CUDA launch per call for one layer (``rdkv_unpack_layer``) and per 16 layers of a
+cache (``rdkv_unpack_layers``).  Tensors must be on a CUDA device.
 """
 from __future__ import annotations
 
@@ -13,7 +14,7 @@ from typing import List, Optional, Tuple
 import torch
 from torch import Tensor
 
-from ._lib import LayerView, check, lib, ptr, require_cuda, stream_ptr
+from ._lib import LayerView, UnpackJob, check, lib, ptr, require_cuda, stream_ptr
 from .packing import PackedKVLayer, TriZoneCache, _squeeze_h, layer_view
 
 
@@ -130,6 +131,98 @@ def _unpack_v_perhead(pl: PackedKVLayer, *, head_dim: int) -> Tensor:
     return _v_stripe(pl, None, head_dim, int(pl.T_eff), with_zone_b=False)
 
 
+def _fill_view(v: LayerView, pl: PackedKVLayer, V16: Optional[Tensor], rows: int) -> Optional[list]:
+    """The fields of ``rdkv_layer_view`` the decompressor reads, straight from a layer whose tensors are
+    ``[1,H_kv,...]`` with contiguous rows (what this library packs); False for any other layer, which takes
+    :func:`rdkv_b200.packing.layer_view`.  Returns the temporaries to keep alive."""
+    def side(name, t, elt):
+        if t is None or t.numel() == 0:
+            return True
+        if t.dim() != 4 or t.shape[0] != 1 or t.stride(3) != 1:
+            return False
+        require_cuda(t, name)
+        setattr(v, name, t.data_ptr())
+        setattr(v, name + "_head_stride", t.stride(1) * elt)
+        return True
+
+    n2c, n4c, n8c = (int(x) for x in pl.K_ch_seg_bounds)
+    v.n_ch2_pad, v.n_ch4_pad, v.n_ch8 = (n2c + 3) // 4 * 4, (n4c + 1) // 2 * 2, n8c
+    ok = (side("k2", pl.K_2bit if n2c else None, 1) and side("k4", pl.K_4bit if n4c else None, 1)
+          and side("k8", pl.K_8bit if n8c else None, 1) and side("v2", pl.V_2bit, 1) and side("v4", pl.V_4bit, 1)
+          and side("v8", pl.V_8bit, 1) and side("v16", V16, 1))
+    ks, kz, vs, vz = pl.K_ch_scale, pl.K_ch_zp, pl.V_scale, pl.V_zp
+    if not ok or not (ks.dim() == kz.dim() == vs.dim() == vz.dim() == 4 and ks.is_contiguous() and kz.is_contiguous()
+                      and vs.shape[3] == vz.shape[3] == 1 and vs.stride(2) == vz.stride(2) == 1 and vs.stride(1) == vz.stride(1)):
+        return None
+    for name, t in (("k_scale", ks), ("k_zp", kz), ("v_scale", vs), ("v_zp", vz)):
+        if t.numel():
+            require_cuda(t, name)
+            setattr(v, name, t.data_ptr())
+    v.v_meta_head_stride = vs.stride(1)
+    keep = []
+
+    def counts(name, t):
+        if t.dtype != torch.int32 or not t.is_contiguous():
+            t = t.to(torch.int32).contiguous()
+        require_cuda(t, name)
+        keep.append(t)
+        setattr(v, name, t.data_ptr())
+
+    if pl.seg_bounds_per_head is not None:
+        counts("v_seg_bounds", pl.seg_bounds_per_head)
+    v.n2, v.n4, v.n8 = (int(x) for x in pl.seg_bounds)
+    v.max_t_v, v.t_k = int(pl.T_eff), rows
+    if V16 is not None and V16.numel() > 0:
+        v.n_v16_shared = int(V16.shape[-2])
+        if pl.n_v16_per_head is not None:
+            counts("n_v16", pl.n_v16_per_head)
+    return keep
+
+
+def _unpack_layers(layers, V16s, D: int) -> List[Tuple[Tensor, Tensor]]:
+    """(K, V) fp16 stripes of every layer, the fp16-V rows included: ``unpack_k_mixed`` and ``_v_stripe``
+    of all of them in one call."""
+    jobs = (UnpackJob * max(1, len(layers)))()
+    out, keep, n = [], [], 0
+    devices = set()
+    for i, (pl, V16) in enumerate(zip(layers, V16s)):
+        if pl.K_ch_scale is None:
+            raise ValueError("unpack_k_mixed: K_ch_scale missing")
+        require_cuda(pl.K_ch_scale, "K_ch_scale")
+        device = pl.K_ch_scale.device
+        H = int(pl.K_ch_scale.shape[1] if pl.K_ch_scale.dim() == 4 and pl.K_ch_scale.shape[0] == 1 else pl.K_ch_scale.shape[0])
+        rows_k = int(pl.T_eff_k) if pl.T_eff_k > 0 else int(pl.T_eff)
+        n16 = int(pl.n_v16) if _is_perhead_layout(pl) else (int(V16.shape[2]) if V16 is not None and V16.numel() > 0 else 0)
+        rows = int(pl.T_eff) + n16
+        assert rows_k == rows, (f"layer {i}: K T-dim {rows_k} != V T-dim {rows} "
+                                f"(T_v={pl.T_eff}, n_v16={pl.n_v16}, T_eff_k={pl.T_eff_k})")
+        si, stride, cnt, n_ch = _k_channel_maps(pl)
+        no_k = si is None or sum(n_ch) == 0
+        K = (torch.zeros if no_k else torch.empty)((1, H, rows, D), dtype=torch.float16, device=device)
+        V = torch.empty((1, H, rows, D), dtype=torch.float16, device=device)
+        out.append((K, V))
+        if rows == 0:
+            continue
+        job = jobs[n]
+        tmp = _fill_view(job.view, pl, V16, rows)
+        if tmp is None:
+            job.view, tmp = layer_view(pl, V16, t_k=rows)
+        keep.append((tmp, si, cnt))
+        if not no_k:
+            job.k_sort_idx, job.k_sort_idx_head_stride, job.k_ch_counts = si.data_ptr(), stride, ptr(cnt)
+            job.n_ch2, job.n_ch4, job.n_ch8 = n_ch
+            job.k_out = K.data_ptr()
+        job.H_kv, job.v_out, job.out_head_stride, job.rows_out = H, V.data_ptr(), rows * D, rows
+        devices.add(device)
+        n += 1
+    for device in devices:
+        stream = stream_ptr(device)
+    if n:
+        check(lib().rdkv_unpack_layers(jobs, n, D, stream), "rdkv_unpack_layers")
+    del keep
+    return out
+
+
 def unpack_trizone_to_past_kv(dual_cache: TriZoneCache, *, head_dim: int, device: Optional[torch.device] = None,
                               dtype: torch.dtype = torch.float16, return_masks: bool = False,
                               H_q: Optional[int] = None, max_new_tokens: int = 0,
@@ -140,24 +233,9 @@ def unpack_trizone_to_past_kv(dual_cache: TriZoneCache, *, head_dim: int, device
     layers).  Same contract as trizone_decompress.py:185-333."""
     past_kv: List[Tuple[Tensor, Tensor]] = []
     masks_list: List[Optional[Tensor]] = []
-    for i, pl in enumerate(dual_cache.packed):
-        K_full = unpack_k_mixed(pl, D=head_dim)
-        V16 = dual_cache.new_v_only[i] if i < len(dual_cache.new_v_only) else None
+    V16s = [dual_cache.new_v_only[i] if i < len(dual_cache.new_v_only) else None for i in range(len(dual_cache.packed))]
+    for i, (pl, (K_full, V_full)) in enumerate(zip(dual_cache.packed, _unpack_layers(dual_cache.packed, V16s, head_dim))):
         per_head = _is_perhead_layout(pl)
-        if per_head:
-            rows = int(pl.T_eff) + int(pl.n_v16)
-            V_full = _v_stripe(pl, V16, head_dim, rows, with_zone_b=True)
-        else:
-            n16 = int(V16.shape[2]) if V16 is not None and V16.numel() > 0 else 0
-            rows = int(pl.T_eff) + n16
-            if rows == 0:
-                V_full = torch.empty(1, K_full.shape[1], 0, head_dim, dtype=torch.float16, device=K_full.device)
-            else:
-                V_full = _v_stripe(pl, V16, head_dim, rows, with_zone_b=True)
-        assert K_full.shape[2] == V_full.shape[2], (
-            f"layer {i}: K T-dim {K_full.shape[2]} != V T-dim {V_full.shape[2]} "
-            f"(T_v={pl.T_eff}, n_v16={pl.n_v16}, T_eff_k={pl.T_eff_k})")
-        assert K_full.shape[3] == head_dim and V_full.shape[3] == head_dim
         if device is not None:
             K_full, V_full = K_full.to(device), V_full.to(device)
         past_kv.append((K_full.to(dtype).contiguous(), V_full.to(dtype).contiguous()))
