@@ -508,6 +508,18 @@ int rdkv_sizeof_pack_job(void);
 int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H, int D, int max_slots,
                          int max_t_k, int max_d_pad, int k_passes, int max_k_quads, void* stream);
 
+/* ── prefill: the K allocation's budgets ──────────────────────────────────────
+ * out[r] = k_budget_bits / (head_dim * max(1, number of v_bits[r][0..len) above 0)), rounded as the
+ * reference's expression is (obkv_fast.py:983, 1033-1035). */
+int rdkv_k_budgets(const int64_t* v_bits, int64_t row_stride, int n_rows, int len, int head_dim,
+                   float k_budget_bits, float* out, void* stream);
+
+/* Bits each of n_layers packed layers stands for (obkv_accel/blockwise_decode.py:665-678): v_bits
+ * [n_layers][H][T], k_bits [n_layers][H][head_dim] -> out [n_layers] = sum(v_bits) * head_dim + sum over heads of
+ * (head's k_bits) * (head's tokens with bits above 0). */
+int rdkv_logical_bits(const int64_t* v_bits, const int64_t* k_bits, int n_layers, int H, int T, int head_dim,
+                      int64_t* out, void* stream);
+
 /* ── prefill: batched Lagrangian bit allocator ────────────────────────────────
  * Replaces knapsack_bit_allocation_batched (knapsack_solver.py:121-248).
  * scores fp32 [n_rows][len] (row_stride elements); budget fp32 [n_rows];
@@ -519,6 +531,11 @@ int rdkv_knapsack_batched(const float* scores, int64_t row_stride, int n_rows, i
                           const float* budget, const float* option_bits, const float* option_eps,
                           int n_options, int max_iters, float tol, int64_t* out, void* scratch,
                           void* stream);
+
+/* The same with one budget for all rows. */
+int rdkv_knapsack_batched_uniform(const float* scores, int64_t row_stride, int n_rows, int len, float budget,
+                                  const float* option_bits, const float* option_eps, int n_options, int max_iters,
+                                  float tol, int64_t* out, void* scratch, void* stream);
 
 /* Single-row form, for any number of independent rows.  Replaces knapsack_bit_allocation
  * (knapsack_solver.py:39-118), whose arithmetic differs from the batched solver's: the multiplier

@@ -9,6 +9,7 @@ per-row freeze) runs inside one kernel pair, one CTA per row.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import json
 from typing import Dict, Optional, Tuple, Union
 
@@ -44,25 +45,35 @@ def knapsack_bit_allocation_batched(scores: torch.Tensor, budget_per_token: Unio
         s = s.contiguous()
     B, T = s.shape
     dev = s.device
+    budget, uniform = None, 0.0
     if torch.is_tensor(budget_per_token):
         assert budget_per_token.shape == (B,), (
             f"budget_per_token tensor must be [B={B}]; got {tuple(budget_per_token.shape)}")
         budget = budget_per_token.detach().float().to(dev).contiguous()
     else:
-        budget = torch.full((B,), float(budget_per_token), dtype=torch.float32, device=dev)
+        uniform = float(budget_per_token)                  # (travels with the launch)
     opt = [float(b) for b in bits.tolist()]
-    eps = [float(epsilon[int(b)]) for b in opt]
-    n = len(opt)
+    n, c_bits, c_eps = _option_arrays(tuple(opt), tuple(float(epsilon[int(b)]) for b in opt))
     out = torch.empty((B, T), dtype=torch.int64, device=dev)
     if B == 0 or T == 0:
         return out
     scratch = torch.empty(3 * B, dtype=torch.int32, device=dev)
-    c_bits = (C.c_float * n)(*opt)
-    c_eps = (C.c_float * n)(*eps)
-    check(lib().rdkv_knapsack_batched(ptr(s), s.stride(0), B, T, ptr(budget), c_bits, c_eps, n, int(max_iters),
-                                      float(tol), ptr(out), ptr(scratch), stream_ptr(dev)),
-          "rdkv_knapsack_batched")
+    if budget is not None:
+        check(lib().rdkv_knapsack_batched(s.data_ptr(), s.stride(0), B, T, budget.data_ptr(), c_bits, c_eps, n, int(max_iters),
+                                          float(tol), out.data_ptr(), scratch.data_ptr(), stream_ptr(dev)),
+              "rdkv_knapsack_batched")
+    else:
+        check(lib().rdkv_knapsack_batched_uniform(s.data_ptr(), s.stride(0), B, T, uniform, c_bits, c_eps, n, int(max_iters),
+                                                  float(tol), out.data_ptr(), scratch.data_ptr(), stream_ptr(dev)),
+              "rdkv_knapsack_batched_uniform")
     return out
+
+
+@functools.lru_cache(maxsize=64)
+def _option_arrays(opt: Tuple[float, ...], eps: Tuple[float, ...]):
+    """Bit options and their distortions as C arrays (read by the launch, not kept by it)."""
+    n = len(opt)
+    return n, (C.c_float * n)(*opt), (C.c_float * n)(*eps)
 
 
 def knapsack_bit_allocation(scores: torch.Tensor, budget_per_token: float,
@@ -140,3 +151,15 @@ def k_average_bits_per_head(token_budget: int, head_dim: int, k_budget_ratio: fl
     fp32 tensor)."""
     k_budget_bits = k_budget_ratio * total_budget_bits(token_budget, head_dim)
     return k_budget_bits / (int(head_dim) * kept_tokens_per_head.clamp(min=1).float())
+
+
+def k_budgets_from_v_bits(token_budget: int, head_dim: int, k_budget_ratio: float, v_bits: torch.Tensor) -> torch.Tensor:
+    """:func:`k_average_bits_per_head` of the tokens kept in every row of ``v_bits`` [H,T] (the V
+    allocation's result on the GPU): the same fp32 values, counted and divided in one launch."""
+    require_cuda(v_bits, "v_bits")
+    H, T = v_bits.shape
+    out = torch.empty(H, dtype=torch.float32, device=v_bits.device)
+    check(lib().rdkv_k_budgets(v_bits.data_ptr(), v_bits.stride(0), H, T, int(head_dim),
+                               k_budget_ratio * total_budget_bits(token_budget, head_dim), out.data_ptr(),
+                               stream_ptr(v_bits.device)), "rdkv_k_budgets")
+    return out

@@ -8,6 +8,53 @@ from helpers import to_np
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("length", [1, 33, 128, 129, 256, 257, 2048, 4096, 8191, 16385, 65537])
+@pytest.mark.parametrize("kind", ["lognormal", "softmax", "ties", "zeros", "negative", "tiny"])
+def test_allocator_lengths(length, kind):
+    """Row lengths at which a row moves from a warp to a CTA and to clusters; rows whose scores sit in a
+    few buckets, on ties, at zero, below it and near the smallest numbers."""
+    from oracle.ref_knapsack import knapsack_batched
+    from rdkv_b200 import synth
+    from rdkv_b200.knapsack_solver import knapsack_bit_allocation_batched
+    gen = torch.Generator().manual_seed(length)
+    s = synth.make_scores(3, length, seed=length)
+    if kind == "softmax":
+        s = torch.softmax(6 * torch.randn(3, length, generator=gen), dim=1)
+    elif kind == "ties":
+        s = torch.randint(0, 4, (3, length), generator=gen).float()
+    elif kind == "zeros":
+        s[:, ::3] = 0.0
+    elif kind == "negative":
+        s = torch.randn(3, length, generator=gen)
+    elif kind == "tiny":
+        s = s * 1e-37
+    for budget, kw in ((2.0, {}), (torch.tensor([0.4, 3.3, 9.0]), dict(max_iters=60)),
+                       (3.0, dict(bit_options=torch.tensor([2.0, 4.0, 8.0])))):
+        got = knapsack_bit_allocation_batched(s.cuda(), budget.cuda() if torch.is_tensor(budget) else budget, epsilon=synth.ALLOC_EPSILON, **kw)
+        want_kw = {k: (v.numpy() if torch.is_tensor(v) else v) for k, v in kw.items()}
+        want = knapsack_batched(s.numpy(), budget.numpy() if torch.is_tensor(budget) else budget, synth.ALLOC_EPSILON, **want_kw)
+        assert np.array_equal(to_np(got), want)
+
+
+@pytest.mark.parametrize("length", [1, 2, 3, 1000, 32768, 40001])
+def test_budgets_and_logical_bits(length):
+    from oracle.ref_blockwise import logical_layer_bits
+    from rdkv_b200 import _lib
+    from rdkv_b200.knapsack_solver import k_average_bits_per_head, k_budgets_from_v_bits
+    gen = torch.Generator().manual_seed(length)
+    bits = torch.tensor([0, 0, 0, 2, 4, 8, 16])[torch.randint(0, 7, (5, length + 1), generator=gen)].cuda()
+    bits[0] = 0
+    for v in (bits, bits[:, 1:]):
+        want = k_average_bits_per_head(777, 128, 0.37, (v > 0).sum(dim=1))
+        assert torch.equal(k_budgets_from_v_bits(777, 128, 0.37, v), want)
+    L, H = 2, 3
+    vb = torch.tensor([0, 2, 4, 8, 16])[torch.randint(0, 5, (L, H, length), generator=gen)].cuda()
+    kb = torch.tensor([0, 2, 4, 8, 16])[torch.randint(0, 5, (L, H, 128), generator=gen)].cuda()
+    out = torch.empty(L, dtype=torch.int64, device="cuda")
+    _lib.check(_lib.lib().rdkv_logical_bits(vb.data_ptr(), kb.data_ptr(), L, H, length, 128, out.data_ptr(), _lib.stream_ptr(out.device)), "logical")
+    assert out.tolist() == [logical_layer_bits(to_np(vb[i]), to_np(kb[i]), 128) for i in range(L)]
+
+
 @pytest.mark.parametrize("rows", [1, 15, 127, 128, 129, 300])
 @pytest.mark.parametrize("mix", [((8, 24), (4, 31), (2, 27)), ((8, 1),), ((4, 2), (2, 126)), ((16, 100), (8, 28))])
 def test_unpack_rows(rows, mix):
