@@ -42,6 +42,7 @@ enum { RDKV_F16 = 0, RDKV_BF16 = 1, RDKV_F32 = 2 };
  * 2 bits), so the kernel that is fast for those is launched.  Results do not depend on it beyond rounding. */
 #define RDKV_K_ANY_ROWS 65536
 
+
 /*
  * One (sequence, layer) of packed cache: H_kv heads in the reference's stacked
  * per-head layout (PackedKVLayer, obkv_accel/packing.py:43-111, plus the fp16
@@ -315,6 +316,32 @@ int rdkv_lse_combine(const float* partials, int64_t n_rows, int n_splits, int64_
 int rdkv_partition_by_bits(const void* bits, int elem_size, int64_t row_stride, int n_rows, int len,
                            int mode, int32_t* order, int32_t* counts, void* stream);
 
+/* A layer's token maps (mode 0) and channel maps (mode 1) in one launch.  counts: [tok_rows + ch_rows][4],
+ * token rows first.  tok_rank ([tok_rows][tok_len], or NULL): for every listed element of the compressed
+ * classes its number among the row's elements with bits > 0 and not 16, in ascending order (the
+ * reference's V sort index, obkv_accel/packing.py:733-735).  fill 0: as mode + 4 above. */
+int rdkv_partition_pair(const void* tok_bits, int tok_elem_size, int64_t tok_row_stride, int tok_rows, int tok_len,
+                        const void* ch_bits, int ch_elem_size, int64_t ch_row_stride, int ch_rows, int ch_len,
+                        int fill, int32_t* tok_order, int32_t* tok_rank, int32_t* ch_order, int32_t* counts,
+                        void* stream);
+
+/* The per-head tables of packed layers from their heads' counts ([H][4], 16-byte aligned): seg_bounds [H][3],
+ * t_eff, n_v16, t_eff_k [H], the additive softmax mask [H*gqa][t_k] (or NULL; obkv_accel/packing.py:
+ * 1236-1257), and sort_idx[i] = rank_row[i] for i < n_sort.  `jobs` is a HOST array (a launch per 8 layers). */
+typedef struct rdkv_pack_meta_job {
+  const int32_t* counts;
+  int32_t* seg_bounds;
+  int32_t* t_eff;
+  int32_t* n_v16;
+  int32_t* t_eff_k;
+  float* mask;
+  const int32_t* rank_row;
+  int64_t* sort_idx;
+  int32_t n_sort, max_t_v, t_k, reserved;
+} rdkv_pack_meta_job;
+int rdkv_sizeof_pack_meta_job(void);
+int rdkv_pack_meta(const rdkv_pack_meta_job* jobs, int n_jobs, int H, int gqa, void* stream);
+
 /* ── prefill: per-token V quantise + bit-pack ─────────────────────────────────
  * Replaces quantize_and_pack(dim=3) + transfer_8bit_to_{2,4}bit_batchwise as
  * used by pack_v_segments (obkv_accel/packing.py:141-165, 715-778;
@@ -507,6 +534,11 @@ int rdkv_sizeof_pack_job(void);
  * units), or 0 for the bound max_d_pad/4 + 2. */
 int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H, int D, int max_slots,
                          int max_t_k, int max_d_pad, int k_passes, int max_k_quads, void* stream);
+/* The same for at most rdkv_pack_inline_jobs() layers whose jobs lie in HOST memory: they travel with the
+ * launches, so there is no device copy of them to wait for or to keep. */
+int rdkv_pack_inline_jobs(void);
+int rdkv_pack_kv_inline(const rdkv_pack_job* jobs_host, int n_jobs, int H, int D, int max_slots,
+                        int max_t_k, int max_d_pad, int k_passes, int max_k_quads, void* stream);
 
 /* ── prefill: the K allocation's budgets ──────────────────────────────────────
  * out[r] = k_budget_bits / (head_dim * max(1, number of v_bits[r][0..len) above 0)), rounded as the
@@ -531,7 +563,6 @@ int rdkv_knapsack_batched(const float* scores, int64_t row_stride, int n_rows, i
                           const float* budget, const float* option_bits, const float* option_eps,
                           int n_options, int max_iters, float tol, int64_t* out, void* scratch,
                           void* stream);
-
 /* The same with one budget for all rows. */
 int rdkv_knapsack_batched_uniform(const float* scores, int64_t row_stride, int n_rows, int len, float budget,
                                   const float* option_bits, const float* option_eps, int n_options, int max_iters,

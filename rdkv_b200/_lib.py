@@ -84,6 +84,15 @@ class PackJob(C.Structure):
 
 _lib: Optional[C.CDLL] = None
 
+class PackMetaJob(C.Structure):
+    """Mirror of ``rdkv_pack_meta_job`` (one layer's per-head tables); field order and types must match the header."""
+    _fields_ = [
+        ("counts", C.c_void_p), ("seg_bounds", C.c_void_p), ("t_eff", C.c_void_p), ("n_v16", C.c_void_p), ("t_eff_k", C.c_void_p),
+        ("mask", C.c_void_p), ("rank_row", C.c_void_p), ("sort_idx", C.c_void_p),
+        ("n_sort", C.c_int32), ("max_t_v", C.c_int32), ("t_k", C.c_int32), ("reserved", C.c_int32),
+    ]
+
+
 class UnpackJob(C.Structure):
     """Mirror of ``rdkv_unpack_job`` (one layer of a batched unpack); field order and types must match the header."""
     _fields_ = [
@@ -136,11 +145,16 @@ _PROTOTYPES = {
     "rdkv_sizeof_unpack_job": ([], _i),
     "rdkv_unpack_layers": ([_p, _i, _i, _p], _i),
     "rdkv_sizeof_pack_job": ([], _i),
+    "rdkv_partition_pair": ([_p, _i, _i64, _i, _i, _p, _i, _i64, _i, _i, _i, _p, _p, _p, _p, _p], _i),
+    "rdkv_sizeof_pack_meta_job": ([], _i),
+    "rdkv_pack_meta": ([_p, _i, _i, _i, _p], _i),
+    "rdkv_pack_inline_jobs": ([], _i),
+    "rdkv_pack_kv_inline": ([_p, _i, _i, _i, _i, _i, _i, _i, _i, _p], _i),
     "rdkv_pack_kv_batched": ([_p, _i, _i, _i, _i, _i, _i, _i, _i, _p], _i),
     "rdkv_k_budgets": ([_p, _i64, _i, _i, _i, _f, _p, _p], _i),
     "rdkv_logical_bits": ([_p, _p, _i, _i, _i, _i, _p, _p], _i),
-    "rdkv_knapsack_batched_uniform": ([_p, _i64, _i, _i, _f, C.POINTER(_f), C.POINTER(_f), _i, _i, _f, _p, _p, _p], _i),
     "rdkv_knapsack_batched": ([_p, _i64, _i, _i, _p, C.POINTER(_f), C.POINTER(_f), _i, _i, _f, _p, _p, _p], _i),
+    "rdkv_knapsack_batched_uniform": ([_p, _i64, _i, _i, _f, C.POINTER(_f), C.POINTER(_f), _i, _i, _f, _p, _p, _p], _i),
     "rdkv_knapsack_rows": ([_p, _i64, _i, _i, _p, C.POINTER(_f), C.POINTER(_f), _i, _i, C.c_double, _p, _p], _i),
     "rdkv_knapsack_static_max_rows": ([], _i),
     "rdkv_knapsack_batched_static": ([_p, _i64, _i, _i, _p, C.POINTER(_f), C.POINTER(_f), _i, _i, _f, _p, _p], _i),
@@ -170,6 +184,8 @@ def lib() -> C.CDLL:
             raise RuntimeError("rdkv_b200: rdkv_tail_args layout mismatch between header and binding")
         if handle.rdkv_sizeof_pack_job() != C.sizeof(PackJob):
             raise RuntimeError("rdkv_b200: rdkv_pack_job layout mismatch between header and binding")
+        if handle.rdkv_sizeof_pack_meta_job() != C.sizeof(PackMetaJob):
+            raise RuntimeError("rdkv_b200: rdkv_pack_meta_job layout mismatch between header and binding")
         if handle.rdkv_sizeof_unpack_job() != C.sizeof(UnpackJob):
             raise RuntimeError("rdkv_b200: rdkv_unpack_job layout mismatch between header and binding")
         _lib = handle

@@ -7,8 +7,8 @@ compressed blocks plus the uncompressed tail (obkv_accel/blockwise_decode.py).  
 
 * ``plan_block_compressions``  — the block schedule (blockwise_decode.py:89-140), host logic;
 * ``_score_block`` / ``_channel_score`` — block scoring on the GPU (:756-810);
-* ``compress_block``           — one block through ``select_and_pack`` per layer, with the
-                                 reference's logical-bit accounting (:812-1121, :659-678);
+* ``compress_block``           — one block through ``select_and_pack``'s steps, all layers
+                                 packed together, with the reference's logical-bit accounting (:812-1121, :659-678);
 * ``multi_source_attention``   — one softmax over any number of packed sources (+ tail) for a
                                  decode step: every source is a view of ONE DecodeTable, the
                                  fused kernel writes a record per (source, head) and the combine
@@ -26,7 +26,7 @@ import torch
 from torch import Tensor
 
 from ._lib import check, lib, ptr, q_dtype_tag, require_cuda, stream_ptr
-from .packing import PackedKVLayer, select_and_pack
+from .packing import PackedKVLayer, _select_bits, pack_selected
 
 
 @dataclass(frozen=True)
@@ -155,30 +155,30 @@ def compress_block(*, target_kv: Sequence[Tensor], query_block: Sequence[Tensor]
     blockwise_decode.py:812-1121, default path): ``target_kv[l]`` [1,H_kv,T,2*D] holds the block's
     keys and values side by side, ``query_block[l]`` [H_q,Q,D] the scoring queries,
     ``token_scores_by_layer[l]`` [H_kv,T] the token scores (from :func:`_score_block`).  Each layer
-    goes through the channel statistic and :func:`rdkv_b200.packing.select_and_pack` with the
-    block's budget; the allocator's decisions are kept on the layer for the bit accounting."""
-    packed_layers, v16_layers, bits = [], [], []
+    goes through the channel statistic and the allocations of
+    :func:`rdkv_b200.packing.select_and_pack` with the block's budget; then all layers are packed
+    together, behind ONE host read of their segment counts.  The allocator's decisions are kept on the
+    layers for the bit accounting."""
     head_dim = int(target_kv[0].shape[-1] // 2)
     h_kv = int(target_kv[0].shape[1])
+    keys, values, v_bits, k_bits = [], [], [], []
     for kv, queries, token_scores in zip(target_kv, query_block, token_scores_by_layer):
-        keys = kv[..., :head_dim].to(dtype=model_dtype)
-        values = kv[..., head_dim:].to(dtype=model_dtype)
-        channel_scores = _channel_score(queries, keys, num_kv_groups=num_kv_groups)
-        packed, new_v_only, _ = select_and_pack(
-            keys, values, token_scores, channel_scores, gqa_factor=num_kv_groups,
-            token_budget=config.block_budget_tokens, k_budget_ratio=config.k_budget_ratio,
-            obs_window=config.obs_window, pool_kernel_size=config.pool_kernel_size,
+        k, v = kv[..., :head_dim].to(dtype=model_dtype), kv[..., head_dim:].to(dtype=model_dtype)
+        channel_scores = _channel_score(queries, k, num_kv_groups=num_kv_groups)
+        vb, kb = _select_bits(
+            k, v, token_scores, channel_scores, token_budget=config.block_budget_tokens,
+            k_budget_ratio=config.k_budget_ratio, pool_kernel_size=config.pool_kernel_size,
             pool_padding=config.pool_padding, pool_type="avg", v_bit_options=config.v_bit_options,
-            k_bit_options=config.k_bit_options, eps_V=config.epsilon_v, eps_K=config.epsilon_k,
-            retain_allocation_metadata=True)
-        if config.correctness_check:
+            k_bit_options=config.k_bit_options, eps_V=config.epsilon_v, eps_K=config.epsilon_k)
+        for every, one in ((keys, k), (values, v), (v_bits, vb), (k_bits, kb)):
+            every.append(one)
+    layers, logical = pack_selected(keys, values, v_bits, k_bits, num_kv_groups)
+    packed_layers, v16_layers = [p for p, _ in layers], [v16 for _, v16 in layers]
+    if config.correctness_check:
+        for packed, new_v_only in layers:
             for t in (packed.K_ch_scale, packed.K_ch_zp, packed.V_scale, packed.V_zp, new_v_only):
                 if t is not None and t.is_floating_point() and not bool(torch.isfinite(t).all()):
                     raise FloatingPointError("non-finite packed metadata")
-        bits.append(_logical_layer_bits_tensor(packed, head_dim))
-        packed_layers.append(packed)
-        v16_layers.append(new_v_only)
-    logical = torch.stack(bits)
     return CompressedDecodeBlock(block_id=block_id, token_start=token_start, token_end=token_end,
                                  packed=tuple(packed_layers), new_v_only=v16_layers, logical_bits_per_layer=logical,
                                  fp16_equivalent_tokens_per_layer=logical.double() / (2 * h_kv * head_dim * 16))

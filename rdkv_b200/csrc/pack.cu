@@ -1,152 +1,17 @@
-// Prefill quantise-and-bitpack: stable partition of the bit maps, per-token V
-// packing and per-channel K packing on the stripe.
+// Prefill quantise-and-bitpack: per-token V packing and per-channel K packing on
+// the stripe (the bit maps' partition: partition.cu).
 //
 // Bit-exactness contract (reference: obkv_accel/packing.py:141-165): fp32 math
 // with one IEEE rounding per operation — true division (__fdiv_rn), no fused
 // multiply-add, round-half-to-even (rintf), fp16 outputs rounded to nearest.
 #include <cooperative_groups.h>
 
+#include <cstring>
 #include <type_traits>
 
 #include "rdkv_common.cuh"
 
 namespace rdkv {
-
-// ───────────────────────────── partition by bits ─────────────────────────────
-constexpr int PART_THREADS = 1024;
-
-__device__ __forceinline__ int64_t load_int(const void* p, int elem_size, int64_t i) {
-  switch (elem_size) {
-    case 1: return reinterpret_cast<const int8_t*>(p)[i];
-    case 2: return reinterpret_cast<const int16_t*>(p)[i];
-    case 4: return reinterpret_cast<const int32_t*>(p)[i];
-    default: return reinterpret_cast<const int64_t*>(p)[i];
-  }
-}
-
-__device__ __forceinline__ int bit_class(int64_t b, int mode) {
-  if (b == 2) return 0;
-  if (b == 4) return 1;
-  if (b == 8) return 2;
-  if (b == 16) return mode == 0 ? 3 : 2;
-  return -1;
-}
-
-__global__ void __launch_bounds__(PART_THREADS)
-partition_kernel(const void* bits, int elem_size, int64_t row_stride, int len, int mode_flags,
-                 int32_t* order, int32_t* counts) {
-  const int mode = mode_flags & 1;                         // (bit 2 of mode_flags: leave the entries past the kept count alone)
-  __shared__ int warp_tot[4][PART_THREADS / 32];
-  __shared__ int class_base[5];
-  const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t off = (int64_t)row * row_stride;
-  const int per = (len + PART_THREADS - 1) / PART_THREADS;
-  const int lo = min(len, tid * per), hi = min(len, lo + per);
-  int cnt[4] = {0, 0, 0, 0};
-  // Up to 32 elements per thread are classified once and remembered as three bit masks (kept, class
-  // bit 0, class bit 1), so the scatter pass below does not read the map again; 16-bit maps whose
-  // per-thread chunks are 16-byte aligned are read with 16-byte loads.
-  const bool cached = per <= 32;
-  uint32_t m_keep = 0u, m_c0 = 0u, m_c1 = 0u;
-  auto note = [&](int k, int64_t b) {
-    const int c = bit_class(b, mode);
-    if (c >= 0) {
-      cnt[c]++;
-      m_keep |= 1u << k; m_c0 |= (uint32_t)(c & 1) << k; m_c1 |= (uint32_t)(c >> 1) << k;
-    }
-  };
-  const bool vec = cached && elem_size == 2 && (per & 7) == 0 && hi - lo == per &&
-                   ((reinterpret_cast<uintptr_t>(bits) + 2 * (off + lo)) & 15) == 0;
-  if (vec) {
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const int16_t*>(bits) + off + lo);
-    uint4 w[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) w[u] = u * 8 < per ? __ldg(src + u) : make_uint4(0u, 0u, 0u, 0u);
-    // 16-bit values without branches: kept = a power of two in [2, 16]; class = log2 - 1 (16 counts as 8
-    // for channel maps); the four class counts (at most 32 each) share one register, 8 bits apiece
-    uint32_t cnt4 = 0u;
-    auto note16 = [&](int k, uint32_t v) {
-      const uint32_t ok = (uint32_t)((v - 2u <= 14u) & ((v & (v - 1u)) == 0u));
-      uint32_t c = (30u - (uint32_t)__clz((int)(v | 1u))) & 3u;
-      if (mode != 0) c = min(c, 2u);
-      cnt4 += ok << (8u * c);
-      m_keep |= ok << k; m_c0 |= (ok & c) << k; m_c1 |= (ok & (c >> 1)) << k;
-    };
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (u * 8 >= per) break;
-      const uint32_t x[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        note16(8 * u + 2 * e, x[e] & 0xFFFFu);
-        note16(8 * u + 2 * e + 1, x[e] >> 16);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) cnt[c] = (int)((cnt4 >> (8 * c)) & 0xFFu);
-  } else if (cached) {
-    for (int i = lo; i < hi; ++i) note(i - lo, load_int(bits, elem_size, off + i));
-  } else {
-    for (int i = lo; i < hi; ++i) {
-      const int c = bit_class(load_int(bits, elem_size, off + i), mode);
-      if (c >= 0) cnt[c]++;
-    }
-  }
-  int excl[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    int v = cnt[c];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int n = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += n;
-    }
-    excl[c] = v - cnt[c];
-    if (lane == 31) warp_tot[c][warp] = v;
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      int v = warp_tot[c][lane];
-      const int own = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += n;
-      }
-      warp_tot[c][lane] = v - own;
-      if (lane == 31) class_base[c + 1] = v;       // class totals (converted to bases below)
-    }
-  }
-  __syncthreads();
-  if (tid == 0) {
-    const int n0 = class_base[1], n1 = class_base[2], n2 = class_base[3], n3 = class_base[4];
-    counts[row * 4 + 0] = n0; counts[row * 4 + 1] = n1; counts[row * 4 + 2] = n2; counts[row * 4 + 3] = n3;
-    class_base[0] = 0; class_base[1] = n0; class_base[2] = n0 + n1; class_base[3] = n0 + n1 + n2;
-    class_base[4] = n0 + n1 + n2 + n3;
-  }
-  __syncthreads();
-  int pos[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) pos[c] = class_base[c] + warp_tot[c][warp] + excl[c];
-  int32_t* orow = order + (int64_t)row * len;
-  if (cached) {
-    for (uint32_t m = m_keep; m != 0u; m &= m - 1) {       // kept elements in ascending order
-      const int k = __ffs(m) - 1;
-      const int c = ((m_c0 >> k) & 1u) | (((m_c1 >> k) & 1u) << 1);
-      orow[pos[c]++] = lo + k;
-    }
-  } else {
-    for (int i = lo; i < hi; ++i) {
-      const int c = bit_class(load_int(bits, elem_size, off + i), mode);
-      if (c >= 0) orow[pos[c]++] = i;
-    }
-  }
-  if (mode_flags & 4) return;
-  const int kept = class_base[4];
-  for (int i = kept + tid; i < len; i += PART_THREADS) orow[i] = -1;
-}
 
 // ───────────────────────────── quantisation core ─────────────────────────────
 struct QParam { float scale, zp, qmax; };
@@ -633,6 +498,8 @@ pack_k_minmax_kernel(PackKArgs A) { pack_k_minmax_body(A, blockIdx.y, blockIdx.x
 __global__ void __launch_bounds__(128)
 pack_k_minmax128_kernel(PackKArgs A) { pack_k_minmax_body128(A, blockIdx.y, blockIdx.x); }
 
+constexpr int PARAM_THREADS = 512;                           // (bound by its chains of loads: every slab's extrema in flight at once)
+
 // Pass 2 (one CTA per head): reduce the slab extrema to scale / zero point per channel slot
 // (kept in fp32 in the head's last scratch block for pass 3) and write the per-head tables.
 __device__ __forceinline__ void pack_k_params_body(const PackKArgs& A, int h) {
@@ -690,20 +557,24 @@ __device__ __forceinline__ void pack_k_params_body(const PackKArgs& A, int h) {
   }
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(PARAM_THREADS)
 pack_k_params_kernel(PackKArgs A) { pack_k_params_body(A, blockIdx.x); }
 
-// Pass 3: quantise and bit-pack.  A CTA takes PACKK_BPC consecutive blocks of PACKK_ROWS stripe rows,
+// Pass 3: quantise and bit-pack.  A CTA takes one to PACKK_BPC consecutive blocks of PACKK_ROWS stripe rows,
 // so the per-head set-up (channel parameters, stripe-row -> token map) is paid once for all of
 // them; each warp stages its own rows of the next block with cp.async while it quantises the
 // current one (two buffers, no CTA-wide barrier in the loop).
 constexpr int PACKK_WARPS = 8;
 constexpr int PACKK_ROWS = 128;                              // stripe rows per block
 constexpr int PACKK_RPW = PACKK_ROWS / PACKK_WARPS;          // rows per warp and block
-constexpr int PACKK_BPC = 4;                                 // blocks per CTA
+constexpr int PACKK_BPC = 4;                                 // blocks per CTA, at most
 
-__host__ __device__ inline int pack_k_quant_ctas(int t_k) {
-  return (t_k + PACKK_ROWS * PACKK_BPC - 1) / (PACKK_ROWS * PACKK_BPC);
+// CTAs per head: as few as give every SM two CTAs (three fit), at most one per block
+__host__ inline int pack_k_quant_ctas(int t_k, int64_t heads) {
+  const int blocks = (t_k + PACKK_ROWS - 1) / PACKK_ROWS;
+  const int64_t wanted = (4 * 148 + heads - 1) / heads, least = (blocks + PACKK_BPC - 1) / PACKK_BPC;
+  const int64_t n = wanted > least ? wanted : least;
+  return (int)(n < blocks ? n : blocks);
 }
 __host__ __device__ inline size_t pack_k_quant_smem(int d_pad, bool staged) {
   return (size_t)d_pad * (3 * sizeof(float)) + (staged ? 16 + 2 * PACKK_ROWS * 128 * sizeof(uint16_t) : 0);
@@ -724,9 +595,10 @@ __device__ __forceinline__ void pack_k_quant_body(const PackKArgs& A, int h, int
   const uint16_t* __restrict__ K = A.K;
   const int t_k = A.t_k, n2p = A.n2p, n4p = A.n4p, n8p = A.n8p, n_slabs = A.n_slabs, ov = A.qbits_override;
   const int64_t rows_k = A.rows_k;
-  const int row_base = block_x * PACKK_ROWS * PACKK_BPC;
+  const int per_cta = ((t_k + PACKK_ROWS - 1) / PACKK_ROWS + (int)gridDim.x - 1) / (int)gridDim.x;   // blocks (the grid is sized for the longest layer)
+  const int row_base = block_x * PACKK_ROWS * per_cta;
   if (row_base >= t_k) return;
-  const int n_blocks = min(PACKK_BPC, (t_k - row_base + PACKK_ROWS - 1) / PACKK_ROWS);
+  const int n_blocks = min(per_cta, (t_k - row_base + PACKK_ROWS - 1) / PACKK_ROWS);
   const int d_pad = n2p + n4p + n8p;
   float* s_scale = reinterpret_cast<float*>(smem_raw);          // [d_pad]
   float* s_zp = s_scale + d_pad;                                 // [d_pad]
@@ -870,7 +742,18 @@ pack_k_quant_kernel(PackKArgs A) {
 }
 
 // ───────────────────────────── all layers in one launch ──────────────────────
-// blockIdx.z = layer; the per-layer arguments come from a device array of jobs.
+// blockIdx.z = layer; the per-layer arguments come from a device array of jobs or, for a few layers, with
+// the launch itself (no copy to wait for, no device memory).
+constexpr int PACK_INLINE_JOBS = 8;
+struct InlineJobs {
+  rdkv_pack_job j[PACK_INLINE_JOBS];
+  __device__ __forceinline__ const rdkv_pack_job& operator[](int i) const { return j[i]; }
+};
+struct JobArray {
+  const rdkv_pack_job* __restrict__ j;
+  __device__ __forceinline__ const rdkv_pack_job& operator[](int i) const { return j[i]; }
+};
+
 __device__ __forceinline__ void job_to_vargs(const rdkv_pack_job& J, PackVArgs& A) {
   A.V = J.V; A.v_head_stride = J.v_head_stride; A.v_row_stride = J.v_row_stride; A.D = J.D;
   A.order = J.tok_order; A.order_row_stride = J.tok_order_row_stride;
@@ -882,8 +765,9 @@ __device__ __forceinline__ void job_to_vargs(const rdkv_pack_job& J, PackVArgs& 
   A.max_t_v = J.max_t_v; A.qbits_override = 0;
 }
 
+template <class Jobs>
 __global__ void __launch_bounds__(PACKV_WARPS * 32)
-pack_v_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
+pack_v_batched_kernel(const __grid_constant__ Jobs jobs) {
   __shared__ float xs[PACKV_WARPS][PACK_MAX_D];
   __shared__ uint8_t cs[PACKV_WARPS][PACK_MAX_D];
   __shared__ PackVArgs A;
@@ -892,8 +776,9 @@ pack_v_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
   pack_v_body(A, blockIdx.y, blockIdx.x, xs, cs);
 }
 
+template <class Jobs>
 __global__ void __launch_bounds__(PACKV_WARPS * 32)
-pack_v128_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
+pack_v128_batched_kernel(const __grid_constant__ Jobs jobs) {
   __shared__ PackVArgs A;
   if (threadIdx.x == 0) job_to_vargs(jobs[blockIdx.z], A);
   __syncthreads();
@@ -913,8 +798,9 @@ __device__ __forceinline__ void job_to_kargs(const rdkv_pack_job& J, PackKArgs& 
   A.stage_rows = (pack_k_fast(J.D, J.k_row_stride, J.K) && (J.k_head_stride & 3) == 0) ? 1 : 0;
 }
 
+template <class Jobs>
 __global__ void __launch_bounds__(128)
-pack_k_minmax_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
+pack_k_minmax_batched_kernel(const __grid_constant__ Jobs jobs) {
   __shared__ PackKArgs A;
   if (threadIdx.x == 0) job_to_kargs(jobs[blockIdx.z], A);
   __syncthreads();
@@ -922,8 +808,9 @@ pack_k_minmax_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
   pack_k_minmax_body(A, blockIdx.y, blockIdx.x);
 }
 
+template <class Jobs>
 __global__ void __launch_bounds__(128)
-pack_k_minmax128_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
+pack_k_minmax128_batched_kernel(const __grid_constant__ Jobs jobs) {
   __shared__ PackKArgs A;
   if (threadIdx.x == 0) job_to_kargs(jobs[blockIdx.z], A);
   __syncthreads();
@@ -934,8 +821,9 @@ pack_k_minmax128_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
     pack_k_minmax_body(A, blockIdx.y, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(128)
-pack_k_params_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
+template <class Jobs>
+__global__ void __launch_bounds__(PARAM_THREADS)
+pack_k_params_batched_kernel(const __grid_constant__ Jobs jobs) {
   __shared__ PackKArgs A;
   if (threadIdx.x == 0) job_to_kargs(jobs[blockIdx.y], A);
   __syncthreads();
@@ -943,8 +831,9 @@ pack_k_params_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
   pack_k_params_body(A, blockIdx.x);
 }
 
+template <class Jobs>
 __global__ void __launch_bounds__(PACKK_WARPS * 32)
-pack_k_quant_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
+pack_k_quant_batched_kernel(const __grid_constant__ Jobs jobs) {
   extern __shared__ __align__(16) unsigned char pk_smem[];
   __shared__ PackKArgs A;
   if (threadIdx.x == 0) job_to_kargs(jobs[blockIdx.z], A);
@@ -967,6 +856,10 @@ pack_k_quant_batched_kernel(const rdkv_pack_job* __restrict__ jobs) {
 constexpr int KOP_CL = 8;
 constexpr int KOP_WARPS = 8;
 constexpr int KOP_MAX_SMEM = 200 * 1024;
+// By itself the one-pass form is taken where two of its CTAs fit an SM: the gather needs the second one's
+// loads in flight.  (4 layers x 8 heads, device time of the K launches: 4096 rows in 75 KB per CTA 27.7 us
+// against 53.3 in three passes, 32 layers 181 against 267; 8192 rows of 92 channels in 190 KB 166 against 109.)
+constexpr int KOP_AUTO_SMEM = 110 * 1024;
 
 __host__ __device__ inline int kop_rows_per_cta(int t_k) { return (((t_k + KOP_CL - 1) / KOP_CL) + 31) & ~31; }
 // (a parked row holds a "quad" of four fp16 values per lane of the quantisation phase: at most
@@ -976,8 +869,9 @@ __host__ __device__ inline size_t kop_smem(int t_k, int d_pad, int quads) {
   return (size_t)d_pad * 20 + 256 + 16 + (size_t)kop_rows_per_cta(t_k) * 8 * quads;
 }
 
+template <class Jobs>
 __global__ void __launch_bounds__(KOP_WARPS * 32, 3)
-pack_k_onepass_batched_kernel(const rdkv_pack_job* __restrict__ jobs, int rows_cap, int quads_cap) {
+pack_k_onepass_batched_kernel(const __grid_constant__ Jobs jobs, int rows_cap, int quads_cap) {
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) unsigned char kop_smem_raw[];
   __shared__ PackKArgs A;
@@ -1221,17 +1115,6 @@ pack_k_onepass_batched_kernel(const rdkv_pack_job* __restrict__ jobs, int rows_c
 
 using namespace rdkv;
 
-extern "C" int rdkv_partition_by_bits(const void* bits, int elem_size, int64_t row_stride, int n_rows,
-                                      int len, int mode, int32_t* order, int32_t* counts, void* stream) {
-  if (bits == nullptr || order == nullptr || counts == nullptr || n_rows < 0 || len < 0) return RDKV_ERR_BAD_ARG;
-  if (elem_size != 1 && elem_size != 2 && elem_size != 4 && elem_size != 8) return RDKV_ERR_BAD_ARG;
-  if ((mode & ~4) != 0 && (mode & ~4) != 1) return RDKV_ERR_BAD_ARG;
-  if (n_rows == 0) return RDKV_OK;
-  partition_kernel<<<n_rows, PART_THREADS, 0, (cudaStream_t)stream>>>(bits, elem_size, row_stride, len, mode,
-                                                                     order, counts);
-  return launch_status();
-}
-
 extern "C" int rdkv_pack_v(const uint16_t* V, int64_t v_head_stride, int64_t v_row_stride, int H, int D,
                            const int32_t* order, int64_t order_row_stride, const int32_t* counts,
                            int64_t counts_row_stride, int n_identity, int identity_bits, int max_n2,
@@ -1305,24 +1188,24 @@ extern "C" int rdkv_pack_k(const uint16_t* K, int64_t k_head_stride, int64_t k_r
     pack_k_minmax_kernel<<<dim3(n_slabs, H), 128, 0, st>>>(A);
   int rc = launch_status();
   if (rc != RDKV_OK) return rc;
-  pack_k_params_kernel<<<H, 128, 0, st>>>(A);
+  pack_k_params_kernel<<<H, PARAM_THREADS, 0, st>>>(A);
   rc = launch_status();
   if (rc != RDKV_OK) return rc;
   const size_t smem = pack_k_quant_smem(d_pad, A.stage_rows != 0);
   if (cudaFuncSetAttribute(pack_k_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return launch_status();
-  pack_k_quant_kernel<<<dim3(pack_k_quant_ctas(t_k), H), PACKK_WARPS * 32, smem, st>>>(A);
+  pack_k_quant_kernel<<<dim3(pack_k_quant_ctas(t_k, H), H), PACKK_WARPS * 32, smem, st>>>(A);
   return launch_status();
 }
 
 extern "C" int rdkv_sizeof_pack_job(void) { return (int)sizeof(rdkv_pack_job); }
 
-extern "C" int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H, int D, int max_slots,
-                                    int max_t_k, int max_d_pad, int k_passes, int max_k_quads, void* stream) {
+template <class Jobs>
+static int pack_kv_jobs(const Jobs& jobs, int n_jobs, int H, int D, int max_slots,
+                        int max_t_k, int max_d_pad, int k_passes, int max_k_quads, void* stream) {
   if (k_passes != 0 && k_passes != 1 && k_passes != 3) return RDKV_ERR_BAD_ARG;
   if (max_k_quads < 0 || max_k_quads > kop_quads_bound(max_d_pad)) return RDKV_ERR_BAD_ARG;
-  if (jobs == nullptr || n_jobs < 0 || H <= 0 || D <= 0 || max_slots < 0 || max_t_k < 0 || max_d_pad < 0)
-    return RDKV_ERR_BAD_ARG;
+  if (n_jobs < 0 || H <= 0 || D <= 0 || max_slots < 0 || max_t_k < 0 || max_d_pad < 0) return RDKV_ERR_BAD_ARG;
   if (D > PACK_MAX_D || (D & 3)) return RDKV_ERR_BAD_SHAPE;
   if (max_d_pad > PACKK_MAX_DPAD) return RDKV_ERR_TOO_LARGE;
   if (n_jobs == 0) return RDKV_OK;
@@ -1330,8 +1213,8 @@ extern "C" int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H
   cudaStream_t st = (cudaStream_t)stream;
   const bool fast = D == 128;
   dim3 gv(pack_v_blocks(max_slots, fast), H, n_jobs);
-  if (fast) pack_v128_batched_kernel<<<gv, PACKV_WARPS * 32, 0, st>>>(jobs);
-  else pack_v_batched_kernel<<<gv, PACKV_WARPS * 32, 0, st>>>(jobs);
+  if (fast) pack_v128_batched_kernel<Jobs><<<gv, PACKV_WARPS * 32, 0, st>>>(jobs);
+  else pack_v_batched_kernel<Jobs><<<gv, PACKV_WARPS * 32, 0, st>>>(jobs);
   int rc = launch_status();
   if (rc != RDKV_OK || max_t_k == 0 || max_d_pad == 0) return rc;
   // K in one pass (the kept rows of a head held in the shared memory of a cluster) where they fit
@@ -1339,8 +1222,8 @@ extern "C" int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H
   const size_t one_smem = kop_smem(max_t_k, max_d_pad, quads);
   const bool one_fits = D == 128 && one_smem <= (size_t)KOP_MAX_SMEM;
   if (k_passes == 1 && !one_fits) return RDKV_ERR_TOO_LARGE;
-  if (one_fits && k_passes != 3) {
-    cudaError_t e = cudaFuncSetAttribute(pack_k_onepass_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (one_fits && (k_passes == 1 || (k_passes == 0 && one_smem <= (size_t)KOP_AUTO_SMEM))) {
+    cudaError_t e = cudaFuncSetAttribute(pack_k_onepass_batched_kernel<Jobs>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)one_smem);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
     cudaLaunchConfig_t cfg = {};
@@ -1353,20 +1236,38 @@ extern "C" int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H
     attr[0].val.clusterDim.x = KOP_CL; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, pack_k_onepass_batched_kernel, jobs, kop_rows_per_cta(max_t_k), quads);
+    e = cudaLaunchKernelEx(&cfg, pack_k_onepass_batched_kernel<Jobs>, jobs, kop_rows_per_cta(max_t_k), quads);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
     return launch_status();
   }
-  if (D == 128) pack_k_minmax128_batched_kernel<<<dim3(pack_k_slabs(max_t_k), H, n_jobs), 128, 0, st>>>(jobs);
-  else pack_k_minmax_batched_kernel<<<dim3(pack_k_slabs(max_t_k), H, n_jobs), 128, 0, st>>>(jobs);
+  if (D == 128) pack_k_minmax128_batched_kernel<Jobs><<<dim3(pack_k_slabs(max_t_k), H, n_jobs), 128, 0, st>>>(jobs);
+  else pack_k_minmax_batched_kernel<Jobs><<<dim3(pack_k_slabs(max_t_k), H, n_jobs), 128, 0, st>>>(jobs);
   rc = launch_status();
   if (rc != RDKV_OK) return rc;
-  pack_k_params_batched_kernel<<<dim3(H, n_jobs), 128, 0, st>>>(jobs);
+  pack_k_params_batched_kernel<Jobs><<<dim3(H, n_jobs), PARAM_THREADS, 0, st>>>(jobs);
   rc = launch_status();
   if (rc != RDKV_OK) return rc;
   const size_t smem = pack_k_quant_smem(max_d_pad, D == 128);
-  if (cudaFuncSetAttribute(pack_k_quant_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(pack_k_quant_batched_kernel<Jobs>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return launch_status();
-  pack_k_quant_batched_kernel<<<dim3(pack_k_quant_ctas(max_t_k), H, n_jobs), PACKK_WARPS * 32, smem, st>>>(jobs);
+  pack_k_quant_batched_kernel<Jobs><<<dim3(pack_k_quant_ctas(max_t_k, (int64_t)H * n_jobs), H, n_jobs), PACKK_WARPS * 32, smem, st>>>(jobs);
   return launch_status();
+}
+
+extern "C" int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H, int D, int max_slots,
+                                    int max_t_k, int max_d_pad, int k_passes, int max_k_quads, void* stream) {
+  if (jobs == nullptr) return RDKV_ERR_BAD_ARG;
+  return pack_kv_jobs(JobArray{jobs}, n_jobs, H, D, max_slots, max_t_k, max_d_pad, k_passes, max_k_quads, stream);
+}
+
+extern "C" int rdkv_pack_inline_jobs(void) { return PACK_INLINE_JOBS; }
+
+extern "C" int rdkv_pack_kv_inline(const rdkv_pack_job* jobs_host, int n_jobs, int H, int D, int max_slots,
+                                   int max_t_k, int max_d_pad, int k_passes, int max_k_quads, void* stream) {
+  if (jobs_host == nullptr || n_jobs < 0) return RDKV_ERR_BAD_ARG;
+  if (n_jobs > PACK_INLINE_JOBS) return RDKV_ERR_TOO_LARGE;
+  InlineJobs inl;
+  memset(&inl, 0, sizeof(inl));
+  memcpy(inl.j, jobs_host, (size_t)n_jobs * sizeof(rdkv_pack_job));
+  return pack_kv_jobs(inl, n_jobs, H, D, max_slots, max_t_k, max_d_pad, k_passes, max_k_quads, stream);
 }

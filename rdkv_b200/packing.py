@@ -108,15 +108,13 @@ def _as_fp16_rows(x: Tensor, name: str) -> Tensor:
     return x
 
 
-def _empty_padded(shape: Sequence[int], dtype: torch.dtype, device) -> Tensor:
-    """Uninitialised tensor whose storage goes on for at least 16 bytes behind its last element.  The decode
+def _empty_padded(shape: Tuple[int, int, int, int], dtype: torch.dtype, device) -> Tensor:
+    """Uninitialised 4-D tensor whose storage goes on for at least 16 bytes behind its last element.  The decode
     kernel copies the 16-byte blocks that cover a range of rows: without the slack the last head's
     blocks would stick out of a tensor whose length is no multiple of 16 bytes (odd channel counts,
     odd row counts), and the launch would have to take slower, guarded copies."""
-    n = 1
-    for x in shape:
-        n *= int(x)
-    return torch.empty(n + 16, dtype=dtype, device=device)[:n].view(*shape)
+    a, b, c, d = shape
+    return torch.empty(a * b * c * d + 16, dtype=dtype, device=device).as_strided((a, b, c, d), (b * c * d, c * d, d, 1))
 
 
 # ── C-ABI wrappers ───────────────────────────────────────────────────────────
@@ -131,19 +129,45 @@ def partition_by_bits(bits: Tensor, mode: int, fill: bool = True) -> Tuple[Tenso
     require_cuda(bits, "bits")
     if bits.dim() != 2:
         raise ValueError("bits must be [rows, len]")
+    bits = _bit_map(bits)
+    R, L = bits.shape
+    order = torch.empty((R, L), dtype=torch.int32, device=bits.device)
+    if not (R and L):
+        return order, torch.zeros((R, 4), dtype=torch.int32, device=bits.device)
+    counts = torch.empty((R, 4), dtype=torch.int32, device=bits.device)
+    check(lib().rdkv_partition_by_bits(ptr(bits), bits.element_size(), bits.stride(0), R, L,
+                                       mode if fill else mode + 4,
+                                       ptr(order), ptr(counts), stream_ptr(bits.device)),
+          "rdkv_partition_by_bits")
+    return order, counts
+
+
+def _bit_map(bits: Tensor) -> Tensor:
+    """A 2-D bit map as the partition kernel reads it: integers of 1 to 8 bytes, contiguous rows."""
     if bits.dtype not in (torch.int8, torch.int16, torch.int32, torch.int64):
         bits = bits.to(torch.int64)
     if bits.stride(1) != 1 and bits.shape[1] > 1:
         bits = bits.contiguous()
-    R, L = bits.shape
-    order = torch.empty((R, L), dtype=torch.int32, device=bits.device)
-    counts = torch.zeros((R, 4), dtype=torch.int32, device=bits.device)
-    if R and L:
-        check(lib().rdkv_partition_by_bits(ptr(bits), bits.element_size(), bits.stride(0), R, L,
-                                           mode if fill else mode + 4,
-                                           ptr(order), ptr(counts), stream_ptr(bits.device)),
-              "rdkv_partition_by_bits")
-    return order, counts
+    return bits
+
+
+def _partition_pair(v_bits: Tensor, k_bits: Tensor):
+    """Token maps [R,T] and channel maps [R,D] in one launch: (token lists [R,T], their ranks among the
+    compressed tokens [R,T], channel lists [R,D], counts [2R,4] with the token rows first).  Entries past
+    a row's kept count are left as they are."""
+    v_bits, k_bits = _bit_map(v_bits), _bit_map(k_bits)
+    (R, T), D = v_bits.shape, k_bits.shape[1]
+    i32 = dict(dtype=torch.int32, device=v_bits.device)
+    tok_order, tok_rank = torch.empty((R, T), **i32), torch.empty((R, T), **i32)
+    ch_order, counts = torch.empty((R, D), **i32), torch.empty((2 * R, 4), **i32)
+    if not (R and T and D):
+        counts = torch.cat([partition_by_bits(v_bits, 0)[1], partition_by_bits(k_bits, 1)[1]])
+    else:
+        check(lib().rdkv_partition_pair(v_bits.data_ptr(), v_bits.element_size(), v_bits.stride(0), R, T,
+                                        k_bits.data_ptr(), k_bits.element_size(), k_bits.stride(0), R, D, 0,
+                                        tok_order.data_ptr(), tok_rank.data_ptr(), ch_order.data_ptr(), counts.data_ptr(),
+                                        stream_ptr(v_bits.device)), "rdkv_partition_pair")
+    return tok_order, tok_rank, ch_order, counts
 
 
 def _launch_pack_v(V: Tensor, order: Optional[Tensor], order_rs: int, counts: Optional[Tensor],
@@ -363,42 +387,138 @@ def pack_kv(K: Tensor, V: Tensor, v_bits: Tensor, k_bits: Tensor, gqa_factor: in
     dev = K.device
     if tuple(v_bits.shape) != (H, T) or tuple(k_bits.shape) != (H, D):
         raise ValueError(f"v_bits must be [{H},{T}] and k_bits [{H},{D}]")
-    tok_order, tok_counts = partition_by_bits(v_bits.to(dev), 0)
-    ch_order, ch_counts = partition_by_bits(k_bits.to(dev), 1)
-    host = torch.cat([tok_counts, ch_counts], dim=0).cpu().tolist()        # the one host read
-    tok_host, ch_host = host[:H], host[H:]
-    mx = [max(r[i] for r in tok_host) for i in range(4)]
-    t_v_h = [r[0] + r[1] + r[2] for r in tok_host]
-    max_t_v, max_n16 = max(t_v_h), mx[3]
-    t_k = max_t_v + max_n16
-    if t_k == 0:
+    v_bits, k_bits = v_bits.to(dev), k_bits.to(dev)
+    parts = _partition_pair(v_bits, k_bits)
+    shape = _PackShapes(parts[3].cpu().numpy(), 1, H)                      # the one host read
+    if int(shape.t_k[0]) == 0:
         raise RuntimeError("pack_kv: every head kept zero tokens")
-    v2, v4, v8, v16, v_scale, v_zp = _launch_pack_v(V, tok_order, tok_order.stride(0), tok_counts, 4, 0, 0,
-                                                    mx, max_t_v)
-    (k2, k4, k8, k_scale, k_zp, sort_ph, perm_ph, perm_q, seg_ch), ch_mx = _pack_k_per_head(
-        K, tok_order, tok_counts, max_t_v, t_k, ch_order, ch_counts, ch_host, gqa_factor)
-    t_v = tok_counts[:, :3].sum(dim=1).to(torch.int32)
-    n16 = tok_counts[:, 3].contiguous()
-    # legacy single-head field: V sort order of the first non-empty head, as ranks inside
-    # that head's compressed-token list
-    h0 = next((h for h in range(H) if t_v_h[h] + tok_host[h][3] > 0), 0)
-    is_comp = (v_bits[h0].to(dev) > 0) & (v_bits[h0].to(dev) != 16)
-    rank = torch.cumsum(is_comp.to(torch.int64), 0) - 1
-    sort_idx = rank[tok_order[h0, :t_v_h[h0]].to(torch.int64)]
-    layer = PackedKVLayer(
-        K_2bit=k2, K_4bit=k4, K_8bit=k8, K_ch_scale=k_scale, K_ch_zp=k_zp,
-        K_ch_sort_idx=sort_ph[0], K_ch_seg_bounds=ch_mx, K_ch_perm_padded_idx=perm_ph[0],
-        V_2bit=v2, V_4bit=v4, V_8bit=v8, V_scale=v_scale, V_zp=v_zp, sort_idx=sort_idx,
-        seg_bounds=(mx[0], mx[1], mx[2]), T_eff=max_t_v,
-        seg_bounds_per_head=tok_counts[:, :3].contiguous(), T_eff_per_head=t_v,
-        softmax_mask=_softmax_mask(t_v, n16, max_t_v, t_k, gqa_factor) if build_mask else None,
-        K_ch_sort_idx_per_head=sort_ph, K_ch_perm_padded_idx_per_head=perm_ph,
-        K_ch_seg_bounds_per_head=seg_ch, K_ch_perm_padded_idx_for_Q=perm_q,
-        T_eff_k=t_k, n_v16=max_n16, T_eff_k_per_head=(t_v + n16).to(torch.int32), n_v16_per_head=n16,
-        allocation_v_bits=v_bits.to(device=dev, dtype=torch.int16) if retain_allocation_metadata else None,
-        allocation_k_bits=k_bits.to(device=dev, dtype=torch.int16) if retain_allocation_metadata else None,
-    )
+    ((layer, v16),) = _pack_exact([K], [V], parts, shape, gqa_factor, build_mask)
+    if retain_allocation_metadata:
+        layer.allocation_v_bits = v_bits.to(dtype=torch.int16)
+        layer.allocation_k_bits = k_bits.to(dtype=torch.int16)
     return layer, v16
+
+
+class _PackShapes:
+    """What the host needs to know of the segment counts of L layers of H heads: ``host`` [2*L*H,4], the
+    token counts of all layers and then their channel counts."""
+
+    def __init__(self, host: np.ndarray, L: int, H: int):
+        self.L, self.H = L, H
+        tok, ch = host[:L * H].reshape(L, H, 4), host[L * H:].reshape(L, H, 4)
+        self.mx = tok.max(axis=1)                                            # [L,4] per-layer segment maxima
+        self.t_v_h = tok[:, :, :3].sum(axis=2)                               # [L,H]
+        self.max_t_v = self.t_v_h.max(axis=1)
+        self.t_k = self.max_t_v + self.mx[:, 3]
+        self.cm = ch[:, :, :3].max(axis=1)                                   # [L,3]
+        self.n2p, self.n4p, self.n8p = (self.cm[:, 0] + 3) // 4 * 4, (self.cm[:, 1] + 1) // 2 * 2, self.cm[:, 2]
+        self.dk = ch[:, :, :3].sum(axis=2).max(axis=1)
+        # the head whose V order is the legacy single-head ``sort_idx``: the first one that kept a token
+        self.h0 = (tok.sum(axis=2) > 0).argmax(axis=1)
+        self.quads = self.n2p // 4 + (self.n4p // 2 + 1) // 2 + (self.n8p + 3) // 4
+
+
+def _layer_tables(counts: Tensor, shape: _PackShapes, layers: Sequence[int], gqa: int, build_mask: bool,
+                  tok_rank: Tensor) -> List[dict]:
+    """The per-head tables of the given layers (one launch), as fields of their PackedKVLayers."""
+    H, T, dev = shape.H, tok_rank.shape[1], counts.device
+    i32 = dict(dtype=torch.int32, device=dev)
+    jobs = (_lib.PackMetaJob * len(layers))()
+    fields = []
+    cnt_p, rank_p = counts.data_ptr(), tok_rank.data_ptr()
+    for J, i in zip(jobs, layers):
+        tv, tk, h0 = int(shape.max_t_v[i]), int(shape.t_k[i]), int(shape.h0[i])
+        n_sort = int(shape.t_v_h[i, h0])
+        seg, t_v, n16, t_eff_k = torch.empty((H, 3), **i32), torch.empty(H, **i32), torch.empty(H, **i32), torch.empty(H, **i32)
+        sort_idx = torch.empty(n_sort, dtype=torch.int64, device=dev)
+        mask = torch.empty((H * gqa, tk), dtype=torch.float32, device=dev) if build_mask and gqa > 0 else None
+        J.counts, J.seg_bounds, J.t_eff, J.n_v16, J.t_eff_k = (cnt_p + i * H * 16, seg.data_ptr(), t_v.data_ptr(), n16.data_ptr(),
+                                                               t_eff_k.data_ptr())
+        J.mask, J.rank_row, J.sort_idx = ptr(mask), rank_p + (i * H + h0) * T * 4, sort_idx.data_ptr()
+        J.n_sort, J.max_t_v, J.t_k = n_sort, tv, tk
+        fields.append(dict(sort_idx=sort_idx, seg_bounds_per_head=seg, T_eff_per_head=t_v, softmax_mask=mask,
+                           T_eff_k_per_head=t_eff_k, n_v16_per_head=n16))
+    check(lib().rdkv_pack_meta(jobs, len(layers), H, max(gqa, 1), stream_ptr(dev)), "rdkv_pack_meta")
+    if build_mask and gqa <= 0:
+        for f, i in zip(fields, layers):
+            f["softmax_mask"] = _softmax_mask(f["T_eff_per_head"], f["n_v16_per_head"], int(shape.max_t_v[i]), int(shape.t_k[i]), gqa)
+    return fields
+
+
+def _pack_exact(Ks: Sequence[Tensor], Vs: Sequence[Tensor], parts, shape: _PackShapes, gqa: int, build_mask: bool,
+                k_passes: int = 0, launch_events: Optional[list] = None) -> List[Tuple[PackedKVLayer, Optional[Tensor]]]:
+    """The packing launches of L layers whose shapes differ (or of one layer): every layer gets tensors of
+    its own size; the jobs go out with the launches, a few layers at a time."""
+    tok_order, tok_rank, ch_order, counts = parts
+    L, H = shape.L, shape.H
+    T, D = Ks[0].shape[2], Ks[0].shape[3]
+    dev = Ks[0].device
+    u8 = dict(dtype=torch.uint8, device=dev)
+    f16 = dict(dtype=torch.float16, device=dev)
+    i64 = dict(dtype=torch.int64, device=dev)
+    tok_p, cnt_p, ch_p = tok_order.data_ptr(), counts.data_ptr(), ch_order.data_ptr()
+    step = int(lib().rdkv_pack_inline_jobs())
+    layers = []
+    mx, cm = shape.mx.tolist(), shape.cm.tolist()
+    t_v_l, t_k_l, dk_l = shape.max_t_v.tolist(), shape.t_k.tolist(), shape.dk.tolist()
+    n2p_l, n4p_l, n8p_l = shape.n2p.tolist(), shape.n4p.tolist(), shape.n8p.tolist()
+    # extrema per slab of rows (the packing in three passes): as many words for every layer
+    words = H * lib().rdkv_pack_k_slabs(max(t_k_l)) * 2 * max(a + b + c for a, b, c in zip(n2p_l, n4p_l, n8p_l))
+    scratch = torch.empty(L * words, dtype=torch.float32, device=dev)
+    scratch_p = scratch.data_ptr()
+    if launch_events is not None:
+        ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+        ev[0].record()
+    for at in range(0, L, step):
+        n = min(step, L - at)
+        jobs = (_lib.PackJob * n)()
+        for i in range(at, at + n):
+            K, V, J = Ks[i], Vs[i], jobs[i - at]
+            m2, m4, m8, m16 = mx[i]
+            tv, tk, dk, n2p, n4p, n8p = t_v_l[i], t_k_l[i], dk_l[i], n2p_l[i], n4p_l[i], n8p_l[i]
+            d_pad = n2p + n4p + n8p
+            v2 = torch.empty((1, H, m2, D // 4), **u8) if m2 else None
+            v4 = torch.empty((1, H, m4, D // 2), **u8) if m4 else None
+            v8 = torch.empty((1, H, m8, D), **u8) if m8 else None
+            v16 = torch.empty((1, H, m16, D), **f16) if m16 else None
+            vs, vz = _empty_padded((1, H, tv, 1), torch.float16, dev), _empty_padded((1, H, tv, 1), torch.float16, dev)
+            k2 = _empty_padded((1, H, tk, n2p // 4), torch.uint8, dev) if n2p else None
+            k4 = _empty_padded((1, H, tk, n4p // 2), torch.uint8, dev) if n4p else None
+            k8 = _empty_padded((1, H, tk, n8p), torch.uint8, dev) if n8p else None
+            ks, kz = torch.empty((1, H, 1, d_pad), **f16), torch.empty((1, H, 1, d_pad), **f16)
+            sort, perm = torch.empty((H, dk), **i64), torch.empty((H, d_pad), **i64)
+            perm_q = torch.empty((H * gqa, d_pad), **i64) if gqa > 0 else None
+            # (without kept channels the K launches have nothing to write)
+            seg = (torch.empty if d_pad else torch.zeros)((H, 3), dtype=torch.int32, device=dev)
+            J.K, J.V = K.data_ptr(), V.data_ptr()
+            J.k_head_stride, J.k_row_stride, J.v_head_stride, J.v_row_stride = K.stride(1), K.stride(2), V.stride(1), V.stride(2)
+            J.tok_order, J.tok_counts = tok_p + i * H * T * 4, cnt_p + i * H * 16
+            J.ch_order, J.ch_counts = ch_p + i * H * D * 4, cnt_p + (L + i) * H * 16
+            J.tok_order_row_stride, J.ch_order_row_stride = T, D
+            J.D, J.gqa = D, max(gqa, 0)
+            J.max_n2, J.max_n4, J.max_n8, J.max_n16, J.max_t_v, J.t_k = m2, m4, m8, m16, tv, tk
+            J.rows2, J.rows4, J.rows8, J.rows16, J.rows_meta, J.rows_k = m2, m4, m8, m16, tv, tk
+            J.n_ch2_pad, J.n_ch4_pad, J.n_ch8, J.d_kept_max = n2p, n4p, n8p, dk
+            J.v2, J.v4, J.v8, J.v16, J.v_scale, J.v_zp = ptr(v2), ptr(v4), ptr(v8), ptr(v16), vs.data_ptr(), vz.data_ptr()
+            J.k2, J.k4, J.k8, J.k_scale, J.k_zp = ptr(k2), ptr(k4), ptr(k8), ks.data_ptr(), kz.data_ptr()
+            J.sort_idx, J.perm, J.perm_q, J.seg_bounds, J.scratch = (sort.data_ptr(), perm.data_ptr(), ptr(perm_q),
+                                                                     seg.data_ptr(), scratch_p + i * words * 4)
+            layers.append((PackedKVLayer(
+                K_2bit=k2, K_4bit=k4, K_8bit=k8, K_ch_scale=ks, K_ch_zp=kz, K_ch_sort_idx=sort[0],
+                K_ch_seg_bounds=tuple(cm[i]),
+                K_ch_perm_padded_idx=perm[0], V_2bit=v2, V_4bit=v4, V_8bit=v8, V_scale=vs, V_zp=vz, sort_idx=None,
+                seg_bounds=(m2, m4, m8), T_eff=tv, K_ch_sort_idx_per_head=sort, K_ch_perm_padded_idx_per_head=perm,
+                K_ch_seg_bounds_per_head=seg, K_ch_perm_padded_idx_for_Q=perm_q, T_eff_k=tk, n_v16=m16), v16))
+        part = slice(at, at + n)
+        check(lib().rdkv_pack_kv_inline(jobs, n, H, D, int(shape.mx[part].sum(axis=1).max()), int(shape.t_k[part].max()),
+                                        int((shape.n2p + shape.n4p + shape.n8p)[part].max()), int(k_passes),
+                                        int(shape.quads[part].max()), stream_ptr(dev)), "rdkv_pack_kv_inline")
+    if launch_events is not None:
+        ev[1].record()
+        launch_events.append(ev)
+    for (layer, _), fields in zip(layers, _layer_tables(counts, shape, range(L), gqa, build_mask, tok_rank)):
+        layer.__dict__.update(fields)
+    return layers
 
 
 class PackedLayerBatch:
@@ -432,6 +552,30 @@ class PackedLayerBatch:
         return (self.layer(i) for i in range(self.n_layers))
 
 
+def _select_bits(K: Tensor, V: Tensor, layer_scores: Tensor, channel_scores: Tensor, *, token_budget: int,
+                 k_budget_ratio: float, pool_kernel_size: int, pool_padding: str, pool_type: str,
+                 v_bit_options: Optional[Tensor], k_bit_options: Optional[Tensor], eps_V: Optional[dict],
+                 eps_K: Optional[dict]) -> Tuple[Tensor, Tensor]:
+    """The allocation half of :func:`select_and_pack`: (v_bits [H_kv,T], k_bits [H_kv,D]), no host read."""
+    from .knapsack_solver import (DEFAULT_EPSILON_K, DEFAULT_EPSILON_V, k_budgets_from_v_bits,
+                                  knapsack_bit_allocation_batched, v_average_bits)
+    from .scoring import apply_score_pooling
+    assert K.dim() == 4 and V.dim() == 4, f"K/V must be [1,H_kv,T,D], got {tuple(K.shape)}/{tuple(V.shape)}"
+    assert layer_scores.dim() == 2, f"layer_scores must be [H_kv,T], got {tuple(layer_scores.shape)}"
+    assert channel_scores.dim() == 2, f"channel_scores must be [H_kv, D], got {tuple(channel_scores.shape)}"
+    require_cuda(K, "K"); require_cuda(layer_scores, "layer_scores"); require_cuda(channel_scores, "channel_scores")
+    T, head_dim = int(layer_scores.shape[1]), int(K.shape[3])
+    pooled = (apply_score_pooling(layer_scores, pool_type, pool_kernel_size, pool_padding)
+              if pool_kernel_size > 1 else layer_scores).float()
+    v_bits = knapsack_bit_allocation_batched(
+        pooled, v_average_bits(token_budget, head_dim, T, k_budget_ratio),
+        epsilon=DEFAULT_EPSILON_V if eps_V is None else eps_V, bit_options=v_bit_options)       # [H_kv,T]
+    k_bits = knapsack_bit_allocation_batched(
+        channel_scores.float(), k_budgets_from_v_bits(token_budget, head_dim, k_budget_ratio, v_bits),
+        epsilon=DEFAULT_EPSILON_K if eps_K is None else eps_K, bit_options=k_bit_options)       # [H_kv,D]
+    return v_bits, k_bits
+
+
 def select_and_pack(K: Tensor, V: Tensor, layer_scores: Tensor, channel_scores: Tensor, *, gqa_factor: int,
                     token_budget: int, k_budget_ratio: float, obs_window: int = 0, pool_kernel_size: int = 5,
                     pool_padding: str = "reflect", pool_type: str = "avg", v_bit_options: Optional[Tensor] = None,
@@ -450,28 +594,43 @@ def select_and_pack(K: Tensor, V: Tensor, layer_scores: Tensor, channel_scores: 
     ``retain_allocation_metadata`` keeps the allocator's decisions on the layer
     (``allocation_v_bits`` / ``allocation_k_bits``), as the blockwise decoder's accounting wants.
     """
-    from .knapsack_solver import (DEFAULT_EPSILON_K, DEFAULT_EPSILON_V, k_average_bits_per_head,
-                                  knapsack_bit_allocation_batched, v_average_bits)
-    from .scoring import apply_score_pooling
-    assert K.dim() == 4 and V.dim() == 4, f"K/V must be [1,H_kv,T,D], got {tuple(K.shape)}/{tuple(V.shape)}"
-    assert layer_scores.dim() == 2, f"layer_scores must be [H_kv,T], got {tuple(layer_scores.shape)}"
-    assert channel_scores.dim() == 2, f"channel_scores must be [H_kv, D], got {tuple(channel_scores.shape)}"
-    require_cuda(K, "K"); require_cuda(layer_scores, "layer_scores"); require_cuda(channel_scores, "channel_scores")
-    H_kv, T = int(layer_scores.shape[0]), int(layer_scores.shape[1])
-    head_dim = int(K.shape[3])
-    pooled = (apply_score_pooling(layer_scores, pool_type, pool_kernel_size, pool_padding)
-              if pool_kernel_size > 1 else layer_scores).float()
-    v_bits = knapsack_bit_allocation_batched(
-        pooled, v_average_bits(token_budget, head_dim, T, k_budget_ratio),
-        epsilon=DEFAULT_EPSILON_V if eps_V is None else eps_V, bit_options=v_bit_options)       # [H_kv,T]
-    kept = (v_bits > 0).sum(dim=1)                                                               # stays on the device
-    k_bits = knapsack_bit_allocation_batched(
-        channel_scores.float(), k_average_bits_per_head(token_budget, head_dim, k_budget_ratio, kept),
-        epsilon=DEFAULT_EPSILON_K if eps_K is None else eps_K, bit_options=k_bit_options)       # [H_kv,D]
-    K = torch.where((k_bits == 0)[None, :, None, :], torch.zeros_like(K), K)                   # evicted channels
+    v_bits, k_bits = _select_bits(K, V, layer_scores, channel_scores, token_budget=token_budget,
+                                  k_budget_ratio=k_budget_ratio, pool_kernel_size=pool_kernel_size,
+                                  pool_padding=pool_padding, pool_type=pool_type, v_bit_options=v_bit_options,
+                                  k_bit_options=k_bit_options, eps_V=eps_V, eps_K=eps_K)
+    # (the reference clears the evicted channels of K here; the packer reads a head's kept channels only)
     layer, new_v_only = pack_kv(K, V, v_bits, k_bits, gqa_factor, build_mask=build_mask,
                                 retain_allocation_metadata=retain_allocation_metadata)
     return layer, new_v_only, int(layer.T_eff)
+
+
+def pack_selected(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Sequence[Tensor], k_bits: Sequence[Tensor],
+                  gqa_factor: int) -> Tuple[List[Tuple[PackedKVLayer, Optional[Tensor]]], Tensor]:
+    """:func:`pack_kv` of several layers (of one shape: together, behind a single host read), with the allocator's
+    decisions kept on the layers (``allocation_v_bits`` / ``allocation_k_bits``), and the bits each of them
+    stands for (int64 [layers], on the device; reference: blockwise_decode.py:665-678)."""
+    L = len(Ks)
+    if any(k.shape != Ks[0].shape for k in Ks):                            # layers of several shapes: one by one
+        each = [pack_selected([k], [v], [vb], [kb], gqa_factor) for k, v, vb, kb in zip(Ks, Vs, v_bits, k_bits)]
+        return [pair for pairs, _ in each for pair in pairs], torch.cat([bits for _, bits in each])
+    Ks, Vs = [_as_fp16_rows(k, "K") for k in Ks], [_as_fp16_rows(v, "V") for v in Vs]
+    H, T, D = Ks[0].shape[1], Ks[0].shape[2], Ks[0].shape[3]
+    for k, v, vb, kb in zip(Ks, Vs, v_bits, k_bits):
+        if tuple(vb.shape) != (H, T) or tuple(kb.shape) != (H, D) or tuple(k.shape) != (1, H, T, D) or k.shape != v.shape:
+            raise ValueError(f"every layer must be [1,{H},{T},{D}] with v_bits [{H},{T}] and k_bits [{H},{D}]")
+    vb, kb = torch.stack(list(v_bits)), torch.stack(list(k_bits))
+    parts = _partition_pair(vb.view(L * H, T), kb.view(L * H, D))
+    logical = torch.empty(L, dtype=torch.int64, device=vb.device)
+    check(lib().rdkv_logical_bits(vb.data_ptr(), kb.data_ptr(), L, H, T, D, logical.data_ptr(), stream_ptr(vb.device)),
+          "rdkv_logical_bits")
+    vb16, kb16 = vb.to(torch.int16), kb.to(torch.int16)
+    shape = _PackShapes(parts[3].cpu().numpy(), L, H)                      # the one host read
+    if int(shape.t_k.min()) == 0:
+        raise RuntimeError("pack_kv: every head kept zero tokens")
+    layers = _pack_exact(Ks, Vs, parts, shape, gqa_factor, True)
+    for i, (layer, _) in enumerate(layers):
+        layer.allocation_v_bits, layer.allocation_k_bits = vb16[i], kb16[i]
+    return layers, logical
 
 
 _PACK_JOB_DTYPE = None
@@ -492,13 +651,13 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
     cache layer by layer: obkv_accel/packing.py:1323-1421, obkv_fast.py:1098-1166).
 
     Ks, Vs: per-layer [1,H_kv,T,D] fp16 tensors; v_bits [L,H_kv,T], k_bits [L,H_kv,D] in
-    {0,2,4,8,16}.  Two partition launches, ONE host read of all segment counts, three
+    {0,2,4,8,16}.  One partition launch, ONE host read of all segment counts, two to four
     packing launches whose third grid dimension is the layer.  Layer ``i`` of the result
     is bit-identical to ``pack_kv(Ks[i], Vs[i], v_bits[i], k_bits[i], gqa_factor)``.
     Layers whose K bit maps lead to different padded channel widths cannot share tall
-    tensors; they are then packed one by one.  ``launch_events``: a list that receives two
-    (start, end) pairs of CUDA events per call, around the two partition launches and around
-    the packing launches (for measurements).  ``k_passes``: 1 = K packed in one pass over the kept
+    tensors; they get tensors of their own, in launches of a few layers each.  ``launch_events``:
+    a list that receives two (start, end) pairs of CUDA events per call, around the partition
+    launch and around the packing launches (for measurements).  ``k_passes``: 1 = K packed in one pass over the kept
     rows (held in the shared memory of a cluster of CTAs; raises if they do not fit), 3 = in three
     (the rows are read twice), 0 = one pass where it fits; the bytes are the same.
     """
@@ -519,29 +678,20 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
     if launch_events is not None:
         pev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
         pev[0].record()
-    tok_order, tok_counts = partition_by_bits(v_bits.reshape(L * H, T), 0, fill=False)   # (read through the counts only)
-    ch_order, ch_counts = partition_by_bits(k_bits.reshape(L * H, D), 1, fill=False)
+    parts = _partition_pair(v_bits.reshape(L * H, T), k_bits.reshape(L * H, D))
+    tok_order, tok_rank, ch_order, counts = parts
     if launch_events is not None:
         pev[1].record()
         launch_events.append(pev)
-    host = torch.cat([tok_counts, ch_counts], dim=0).cpu().numpy()          # the one host read
-    tok_h = host[:L * H].reshape(L, H, 4)
-    ch_h = host[L * H:].reshape(L, H, 4)
-    mx = tok_h.max(axis=1)                                                   # [L,4] per-layer segment maxima
-    t_v_h = tok_h[:, :, :3].sum(axis=2)                                      # [L,H]
-    max_t_v = t_v_h.max(axis=1)
-    t_k = max_t_v + mx[:, 3]
-    if int(t_k.min()) == 0:
+    shape = _PackShapes(counts.cpu().numpy(), L, H)                         # the one host read
+    if int(shape.t_k.min()) == 0:
         raise RuntimeError("pack_kv_layers: a layer kept zero tokens in every head")
-    cm = ch_h[:, :, :3].max(axis=1)                                          # [L,3]
-    n2p = (cm[:, 0] + 3) // 4 * 4
-    n4p = (cm[:, 1] + 1) // 2 * 2
-    n8p = cm[:, 2]
-    dk = ch_h[:, :, :3].sum(axis=2).max(axis=1)
+    mx, max_t_v, t_k, cm, n2p, n4p, n8p, dk = (shape.mx, shape.max_t_v, shape.t_k, shape.cm, shape.n2p, shape.n4p,
+                                               shape.n8p, shape.dk)
     batch = PackedLayerBatch(L)
     uniform = (n2p == n2p[0]).all() and (n4p == n4p[0]).all() and (n8p == n8p[0]).all() and (dk == dk[0]).all()
     if not uniform or int(n2p[0] + n4p[0] + n8p[0]) == 0:
-        done = [pack_kv(Ks[i], Vs[i], v_bits[i], k_bits[i], gqa_factor, build_mask=build_mask) for i in range(L)]
+        done = _pack_exact(Ks, Vs, parts, shape, gqa_factor, build_mask, k_passes, launch_events)
         batch._make = lambda i: done[i]
         return batch
     N2P, N4P, N8P, DK = int(n2p[0]), int(n4p[0]), int(n8p[0]), int(dk[0])
@@ -578,7 +728,8 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
             "k2": span(K2), "k4": span(K4), "k8": span(K8), "k_scale": span(KS), "k_zp": span(KZ),
             "sort_idx": span(SORT), "perm": span(PERM), "perm_q": span(PERMQ), "seg_bounds": span(SEG),
             "scratch": span(SCR)}
-    to_p, tc_p, co_p, cc_p = tok_order.data_ptr(), tok_counts.data_ptr(), ch_order.data_ptr(), ch_counts.data_ptr()
+    to_p, tc_p, co_p = tok_order.data_ptr(), counts.data_ptr(), ch_order.data_ptr()
+    cc_p = tc_p + L * H * 16
     # the job table, column by column (a numpy record array with the layout of rdkv_pack_job)
     jobs = np.zeros(L, dtype=_pack_job_dtype())
     layer_idx = np.arange(L, dtype=np.int64)
@@ -603,7 +754,7 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
         ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
         ev[0].record()
     check(lib().rdkv_pack_kv_batched(jobs_dev.data_ptr(), L, H, D, int(mx.sum(axis=1).max()), RK, d_pad,
-                                     int(k_passes), N2P // 4 + (N4P // 2 + 1) // 2 + (N8P + 3) // 4, stream_ptr(dev)),
+                                     int(k_passes), int(shape.quads[0]), stream_ptr(dev)),
           "rdkv_pack_kv_batched")
     if launch_events is not None:
         ev[1].record()
@@ -618,25 +769,15 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
         def cut(t: Optional[Tensor], rows: int) -> Optional[Tensor]:
             return None if (t is None or rows == 0) else t[i:i + 1, :, :rows]
 
-        cnt = tok_counts[i * H:(i + 1) * H]
-        t_v = cnt[:, :3].sum(dim=1).to(torch.int32)
-        n16 = cnt[:, 3].contiguous()
-        order_i = tok_order[i * H:(i + 1) * H]
-        h0 = next((h for h in range(H) if int(t_v_h[i, h]) + int(tok_h[i, h, 3]) > 0), 0)
-        is_comp = (v_bits[i, h0] > 0) & (v_bits[i, h0] != 16)
-        rank = torch.cumsum(is_comp.to(torch.int64), 0) - 1
-        sort_idx = rank[order_i[h0, :int(t_v_h[i, h0])].to(torch.int64)]
         layer = PackedKVLayer(
             K_2bit=cut(K2, tk), K_4bit=cut(K4, tk), K_8bit=cut(K8, tk), K_ch_scale=KS[i:i + 1], K_ch_zp=KZ[i:i + 1],
             K_ch_sort_idx=SORT[i, 0], K_ch_seg_bounds=(int(cm[i, 0]), int(cm[i, 1]), int(cm[i, 2])),
             K_ch_perm_padded_idx=PERM[i, 0],
             V_2bit=cut(V2, m2), V_4bit=cut(V4, m4), V_8bit=cut(V8, m8), V_scale=VS[i:i + 1, :, :tv], V_zp=VZ[i:i + 1, :, :tv],
-            sort_idx=sort_idx, seg_bounds=(m2, m4, m8), T_eff=tv,
-            seg_bounds_per_head=cnt[:, :3].contiguous(), T_eff_per_head=t_v,
-            softmax_mask=_softmax_mask(t_v, n16, tv, tk, gqa_factor) if build_mask else None,
+            seg_bounds=(m2, m4, m8), T_eff=tv,
             K_ch_sort_idx_per_head=SORT[i], K_ch_perm_padded_idx_per_head=PERM[i],
             K_ch_seg_bounds_per_head=SEG[i], K_ch_perm_padded_idx_for_Q=PERMQ[i],
-            T_eff_k=tk, n_v16=m16, T_eff_k_per_head=(t_v + n16).to(torch.int32), n_v16_per_head=n16,
+            T_eff_k=tk, n_v16=m16, **_layer_tables(counts, shape, [i], gqa_factor, build_mask, tok_rank)[0],
         )
         return layer, cut(V16, m16)
 
@@ -870,20 +1011,23 @@ def _squeeze_h(t: Optional[Tensor]) -> Optional[Tensor]:
     return t
 
 
+_IDENTITY_FIELDS = ("K_2bit", "K_4bit", "K_8bit", "K_ch_scale", "K_ch_zp", "K_ch_perm_padded_idx_for_Q",
+                    "K_ch_perm_padded_idx_per_head", "K_ch_perm_padded_idx", "V_2bit", "V_4bit", "V_8bit", "V_scale", "V_zp",
+                    "seg_bounds_per_head", "n_v16_per_head", "softmax_mask")
+
+
 def layer_identity(pl) -> tuple:
     """Identity of everything a cached ``rdkv_layer_view`` of this layer captures: address and
     shape of every tensor field it points into and the host scalars it copies.  A cache of views
     keyed by this notices a field that was re-assigned (a deferred K filled in later, a re-pack, a
     grown ``T_eff``); values rewritten in place keep the key, and are read by the kernels anyway."""
-    def ident(t):
-        return None if t is None else (t.data_ptr(), tuple(t.shape), tuple(t.stride()))
-    tensors = tuple(ident(getattr(pl, f, None)) for f in (
-        "K_2bit", "K_4bit", "K_8bit", "K_ch_scale", "K_ch_zp", "K_ch_perm_padded_idx_for_Q",
-        "K_ch_perm_padded_idx_per_head", "K_ch_perm_padded_idx", "V_2bit", "V_4bit", "V_8bit", "V_scale", "V_zp",
-        "seg_bounds_per_head", "n_v16_per_head", "softmax_mask"))
+    tensors = []
+    for f in _IDENTITY_FIELDS:
+        t = getattr(pl, f, None)
+        tensors.append(None if t is None else (t.data_ptr(), t.shape, t.stride()))
     scalars = (tuple(int(x) for x in pl.K_ch_seg_bounds), tuple(int(x) for x in pl.seg_bounds),
                int(pl.T_eff), int(pl.T_eff_k), int(pl.n_v16))
-    return tensors + scalars
+    return tuple(tensors) + scalars
 
 
 def layer_view(pl: PackedKVLayer, V16: Optional[Tensor] = None, n_v16_per_head: Optional[Tensor] = None,

@@ -1,11 +1,45 @@
-"""Prefill kernels at the sizes where they change their way of working, against the oracle, bit for bit."""
+"""Prefill kernels at the sizes where they change their way of working: partition (tiles of 256 elements,
+eight in registers, clusters of CTAs), allocator (a warp per short row, clusters and buckets for long ones),
+batched packing of layers of different shapes, budgets, unpacking; against the oracle, bit for bit."""
 import numpy as np
 import pytest
 import torch
 
-from helpers import to_np
+from helpers import cuda, layer_to_np, to_np
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("length", [1, 7, 255, 256, 257, 4096, 4097, 32769, 131072, 263000])
+@pytest.mark.parametrize("dtype", [torch.int8, torch.int16, torch.int32, torch.int64])
+def test_partition(length, dtype):
+    from rdkv_b200.packing import _partition_pair, partition_by_bits
+    rng = np.random.default_rng(length)
+    rows = 3
+    tok = rng.choice([0, 0, 2, 4, 8, 16, 1, -2, 3], size=(rows, length + 1))
+    if dtype == torch.int64 and length > 2:
+        tok[0, 1], tok[1, 1] = (1 << 32) + 4, -(1 << 33) + 2                 # the low word of neither counts
+    ch = rng.choice([0, 2, 4, 8, 16], size=(rows, 128))
+    maps = torch.from_numpy(tok).to(dtype).cuda()[:, 1:]                     # rows off 16-byte boundaries
+    for mode, bits in ((0, maps), (1, maps)):
+        order, counts = partition_by_bits(bits, mode)
+        for r in range(rows):
+            row = to_np(bits[r]).astype(np.int64)
+            cls = [np.flatnonzero(row == b) for b in (2, 4, 8, 16)]
+            if mode == 1:
+                cls = cls[:2] + [np.flatnonzero((row == 8) | (row == 16)), np.zeros(0, np.int64)]
+            want = np.concatenate(cls)
+            assert to_np(counts[r]).tolist() == [len(c) for c in cls]
+            assert np.array_equal(to_np(order[r])[:len(want)], want) and (to_np(order[r])[len(want):] == -1).all()
+    t_order, t_rank, c_order, counts = _partition_pair(maps, cuda(ch))
+    for r in range(rows):
+        row = to_np(maps[r]).astype(np.int64)
+        want = np.concatenate([np.flatnonzero(row == b) for b in (2, 4, 8, 16)])
+        n_comp = int(np.isin(row, (2, 4, 8)).sum())
+        assert np.array_equal(to_np(t_order[r])[:len(want)], want)
+        rank = np.cumsum((row > 0) & (row != 16)) - 1                        # (every positive value but 16, as the reference counts)
+        assert np.array_equal(to_np(t_rank[r])[:n_comp], rank[want[:n_comp]])
+        assert to_np(counts[rows + r]).tolist() == [int((ch[r] == 2).sum()), int((ch[r] == 4).sum()), int(np.isin(ch[r], (8, 16)).sum()), 0]
 
 
 @pytest.mark.parametrize("length", [1, 33, 128, 129, 256, 257, 2048, 4096, 8191, 16385, 65537])
@@ -53,6 +87,41 @@ def test_budgets_and_logical_bits(length):
     out = torch.empty(L, dtype=torch.int64, device="cuda")
     _lib.check(_lib.lib().rdkv_logical_bits(vb.data_ptr(), kb.data_ptr(), L, H, length, 128, out.data_ptr(), _lib.stream_ptr(out.device)), "logical")
     assert out.tolist() == [logical_layer_bits(to_np(vb[i]), to_np(kb[i]), 128) for i in range(L)]
+
+
+@pytest.mark.parametrize("layers", [1, 3, 9])
+@pytest.mark.parametrize("strided", [False, True])
+def test_layers_of_different_shapes(layers, strided):
+    """Layers whose channel counts differ go out together, a few per launch; every layer equals the
+    oracle's.  Strided: keys and values as halves of one tensor, rows off 16-byte boundaries."""
+    from oracle import ref_packing as RP
+    from rdkv_b200 import synth
+    from rdkv_b200.packing import pack_kv_layers
+    H, T, g = 2, 515, 4
+    Ks, Vs, vbs, kbs = [], [], [], []
+    for i in range(layers):
+        K, V = synth.make_kv(H, T, seed=i)
+        if strided:
+            both = torch.zeros(1, H, T, 259, dtype=torch.float16)
+            both[..., 1:129], both[..., 130:258] = K, V
+            both = both.cuda()
+            Ks.append(both[..., 1:129]); Vs.append(both[..., 130:258])
+        else:
+            Ks.append(K.cuda()); Vs.append(V.cuda())
+        vbs.append(synth.make_v_bits(H, T, 200 + 3 * i, seed=i, per_head_N=[200 + 3 * i, 5 + i]))
+        kbs.append(synth.make_k_bits(H, seed=i, mix=((8, 5 + 3 * i), (4, 20 + i), (2, 30 - i))))
+    batch = pack_kv_layers(Ks, Vs, torch.stack(vbs).cuda(), torch.stack(kbs).cuda(), g)
+    for i, (pl, nv) in enumerate(batch):
+        want, want_nv = RP.pack_kv(to_np(Ks[i]), to_np(Vs[i]), vbs[i].numpy(), kbs[i].numpy(), g)
+        got = layer_to_np(pl)
+        for name in ("K_2bit", "K_4bit", "K_8bit", "K_ch_scale", "K_ch_zp", "V_2bit", "V_4bit", "V_8bit", "V_scale", "V_zp",
+                     "softmax_mask", "seg_bounds_per_head", "n_v16_per_head", "T_eff_per_head", "K_ch_perm_padded_idx_for_Q"):
+            a, b = got[name], want[name]
+            assert (a is None and b is None) or np.array_equal(a, b), (i, name)
+        row = vbs[i][0].numpy()                                              # the first head's V order among its compressed tokens
+        rank = np.cumsum((row > 0) & (row != 16)) - 1
+        assert np.array_equal(got["sort_idx"], rank[np.concatenate([np.flatnonzero(row == b) for b in (2, 4, 8)])])
+        assert np.array_equal(to_np(nv), want_nv)
 
 
 @pytest.mark.parametrize("rows", [1, 15, 127, 128, 129, 300])
