@@ -103,6 +103,7 @@ class DecodeTable:
         # item counters of the persistent form: a pair per launch that may be in flight at the same time
         self.work_ctr = torch.zeros(2 * self.WORK_CTR_SLOTS, dtype=torch.int32, device=self.device)
         self._ws = {}
+        self._plans: dict = {}                              # launch shape -> plan (a pure function of both; see plan())
         # live_counts: the kernel reads the layers' count / scale / permutation tensors itself at every
         # launch (no snapshot to refresh; one more round trip per CTA)
         self.live_counts = bool(live_counts)
@@ -169,6 +170,15 @@ class DecodeTable:
         in k chunks (few units); full rounds of whole units followed by the leftover units cut
         finely enough to fill one more round."""
         rows = self.unit_rows if rows is None else max(64, ((rows + 63) // 64) * 64)
+        key = (n_views, rows, self.n_chunks, self.chunk_rows, self.persistent, self._can_persist())
+        found = self._plans.get(key)
+        if found is None:
+            if len(self._plans) >= 64:                      # (a caller that keeps changing the shape of its launches)
+                self._plans.clear()
+            found = self._plans[key] = self._plan(n_views, rows)
+        return found
+
+    def _plan(self, n_views: int, rows: int):
         units = max(1, n_views * self.H_kv * self._n_hgrp)
         if self.n_chunks is not None:
             k = max(1, min(self.n_chunks, -(-rows // 64)))
@@ -330,7 +340,9 @@ def _launch_units(q: Tensor, table: DecodeTable, out: Optional[Tensor], v0: int 
           else lib().rdkv_decode_attn_persistent if persistent else lib().rdkv_decode_attn)
     extra = (table.work_ctr.data_ptr() + 8 * ctr_slot,) if persistent else ()
     tail_arg = ()
-    if tail is not None:                                   # this range's views of the per-view tail tensors
+    if tail is not None and v0 == 0:
+        tail_arg = (C.byref(tail),)
+    elif tail is not None:                                 # this range's views of the per-view tail tensors
         es = 2
         tv = TailArgs.from_buffer_copy(tail)
         for name, per_view in (("new_k", tv.view_stride * es), ("new_v", tv.view_stride * es),
@@ -341,17 +353,19 @@ def _launch_units(q: Tensor, table: DecodeTable, out: Optional[Tensor], v0: int 
             if base:
                 setattr(tv, name, base + v0 * per_view)
         tail_arg = (C.byref(tv),)
-    with torch.cuda.device(table.device):
-        check(fn(table.views.data_ptr() + v0 * C.sizeof(LayerView), v1 - v0,
-                                     off(q, HEAD_DIM), q_dtype_tag(q), table.H_q, table.H_kv, rows_k, k, n_whole, r0, r1, sp_i, sp_n,
-                                     table.k_rows_arg,
-                                     None if table.live_counts else table.unit_recs.data_ptr() + v0 * table.H_kv * table._unit_rec_bytes,
-                                     None if table.live_counts else table.k_slots.data_ptr() + v0 * table.H_kv * table._k_slot_bytes,
-                                     0 if table.live_counts else table.nkb_max,
-                                     off(ws, k * PARTIAL_STRIDE), table.unit_ctr.data_ptr() + v0 * hy * 4, *extra,
-                                     off(out, HEAD_DIM), off(out_record, PARTIAL_STRIDE),
-                                     ptr(table.status), *tail_arg, stream_ptr(table.device)),
-              "rdkv_decode_attn")
+    unit0 = v0 * table.H_kv
+    args = (table.views.data_ptr() + v0 * C.sizeof(LayerView), v1 - v0, off(q, HEAD_DIM), q_dtype_tag(q), table.H_q, table.H_kv,
+            rows_k, k, n_whole, r0, r1, sp_i, sp_n, table.k_rows_arg,
+            None if table.live_counts else table.unit_recs.data_ptr() + unit0 * table._unit_rec_bytes,
+            None if table.live_counts else table.k_slots.data_ptr() + unit0 * table._k_slot_bytes,
+            0 if table.live_counts else table.nkb_max,
+            off(ws, k * PARTIAL_STRIDE), table.unit_ctr.data_ptr() + v0 * hy * 4, *extra, off(out, HEAD_DIM),
+            off(out_record, PARTIAL_STRIDE), table.status.data_ptr(), *tail_arg)
+    if table.device.index == torch.cuda.current_device():
+        check(fn(*args, stream_ptr(table.device)), "rdkv_decode_attn")
+    else:
+        with torch.cuda.device(table.device):
+            check(fn(*args, stream_ptr(table.device)), "rdkv_decode_attn")
 
 
 _ELEM_SIZE = {0: 2, 1: 2, 2: 4}                           # bytes per element of RDKV_F16 / RDKV_BF16 / RDKV_F32

@@ -135,24 +135,22 @@ def _fill_view(v: LayerView, pl: PackedKVLayer, V16: Optional[Tensor], rows: int
     """The fields of ``rdkv_layer_view`` the decompressor reads, straight from a layer whose tensors are
     ``[1,H_kv,...]`` with contiguous rows (what this library packs); False for any other layer, which takes
     :func:`rdkv_b200.packing.layer_view`.  Returns the temporaries to keep alive."""
-    def side(name, t, elt):
+    n2c, n4c, n8c = pl.K_ch_seg_bounds
+    v.n_ch2_pad, v.n_ch4_pad, v.n_ch8 = (n2c + 3) // 4 * 4, (n4c + 1) // 2 * 2, n8c
+    for name, stride_name, t in (("k2", "k2_head_stride", pl.K_2bit if n2c else None), ("k4", "k4_head_stride", pl.K_4bit if n4c else None),
+                                 ("k8", "k8_head_stride", pl.K_8bit if n8c else None), ("v2", "v2_head_stride", pl.V_2bit),
+                                 ("v4", "v4_head_stride", pl.V_4bit), ("v8", "v8_head_stride", pl.V_8bit),
+                                 ("v16", "v16_head_stride", V16)):
         if t is None or t.numel() == 0:
-            return True
+            continue
         if t.dim() != 4 or t.shape[0] != 1 or t.stride(3) != 1:
-            return False
+            return None
         require_cuda(t, name)
         setattr(v, name, t.data_ptr())
-        setattr(v, name + "_head_stride", t.stride(1) * elt)
-        return True
-
-    n2c, n4c, n8c = (int(x) for x in pl.K_ch_seg_bounds)
-    v.n_ch2_pad, v.n_ch4_pad, v.n_ch8 = (n2c + 3) // 4 * 4, (n4c + 1) // 2 * 2, n8c
-    ok = (side("k2", pl.K_2bit if n2c else None, 1) and side("k4", pl.K_4bit if n4c else None, 1)
-          and side("k8", pl.K_8bit if n8c else None, 1) and side("v2", pl.V_2bit, 1) and side("v4", pl.V_4bit, 1)
-          and side("v8", pl.V_8bit, 1) and side("v16", V16, 1))
+        setattr(v, stride_name, t.stride(1))
     ks, kz, vs, vz = pl.K_ch_scale, pl.K_ch_zp, pl.V_scale, pl.V_zp
-    if not ok or not (ks.dim() == kz.dim() == vs.dim() == vz.dim() == 4 and ks.is_contiguous() and kz.is_contiguous()
-                      and vs.shape[3] == vz.shape[3] == 1 and vs.stride(2) == vz.stride(2) == 1 and vs.stride(1) == vz.stride(1)):
+    if not (ks.dim() == kz.dim() == vs.dim() == vz.dim() == 4 and ks.is_contiguous() and kz.is_contiguous()
+            and vs.shape[3] == vz.shape[3] == 1 and vs.stride(2) == vz.stride(2) == 1 and vs.stride(1) == vz.stride(1)):
         return None
     for name, t in (("k_scale", ks), ("k_zp", kz), ("v_scale", vs), ("v_zp", vz)):
         if t.numel():
@@ -161,21 +159,17 @@ def _fill_view(v: LayerView, pl: PackedKVLayer, V16: Optional[Tensor], rows: int
     v.v_meta_head_stride = vs.stride(1)
     keep = []
 
-    def counts(name, t):
-        if t.dtype != torch.int32 or not t.is_contiguous():
-            t = t.to(torch.int32).contiguous()
-        require_cuda(t, name)
-        keep.append(t)
-        setattr(v, name, t.data_ptr())
-
-    if pl.seg_bounds_per_head is not None:
-        counts("v_seg_bounds", pl.seg_bounds_per_head)
-    v.n2, v.n4, v.n8 = (int(x) for x in pl.seg_bounds)
-    v.max_t_v, v.t_k = int(pl.T_eff), rows
     if V16 is not None and V16.numel() > 0:
         v.n_v16_shared = int(V16.shape[-2])
-        if pl.n_v16_per_head is not None:
-            counts("n_v16", pl.n_v16_per_head)
+    for name, t in (("v_seg_bounds", pl.seg_bounds_per_head), ("n_v16", pl.n_v16_per_head if v.n_v16_shared else None)):
+        if t is not None:
+            if t.dtype != torch.int32 or not t.is_contiguous():
+                t = t.to(torch.int32).contiguous()
+                keep.append(t)
+            require_cuda(t, name)
+            setattr(v, name, t.data_ptr())
+    v.n2, v.n4, v.n8 = (int(x) for x in pl.seg_bounds)
+    v.max_t_v, v.t_k = int(pl.T_eff), rows
     return keep
 
 
@@ -238,7 +232,9 @@ def unpack_trizone_to_past_kv(dual_cache: TriZoneCache, *, head_dim: int, device
         per_head = _is_perhead_layout(pl)
         if device is not None:
             K_full, V_full = K_full.to(device), V_full.to(device)
-        past_kv.append((K_full.to(dtype).contiguous(), V_full.to(dtype).contiguous()))
+        if dtype != torch.float16:
+            K_full, V_full = K_full.to(dtype), V_full.to(dtype)
+        past_kv.append((K_full, V_full))                   # (contiguous: allocated as they are)
         if return_masks:
             if per_head and pl.softmax_mask is not None:
                 mask_2d = pl.softmax_mask
