@@ -16,6 +16,7 @@
 // Probabilities never leave registers.  Zero points are handled outside the products:
 // sum_c zp*q*scale once per CTA (K side, reference "bias trick",
 // obkv_accel/triton_k_kernel.py:14-16) and sum_t p*scale*zp per head (V side).
+#include <cooperative_groups.h>
 #include <cuda.h>   // CUtensorMap (the V tiles arrive through tensor maps; the encoder is looked up through the runtime)
 
 #include <algorithm>
@@ -600,6 +601,27 @@ __device__ __noinline__ void chunk_merge(const float* partials, int* counter, in
   }
 }
 
+// MODE_WEIGHTS with a unit in chunks: the chunks are the CTAs of a cluster, each with its plain sums in its
+// own shared memory; the first adds them up in chunk order.  No workspace and no counters, so that calls on
+// one layer from several streams do not meet.
+__device__ __noinline__ void cluster_sum(float* mine, int gcnt, int n_chunks, float* out_rows) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();                                          // every chunk's sums are in place
+  if (cluster.block_rank() == 0) {
+    for (int i = threadIdx.x; i < gcnt * (D / 4); i += CTA_THREADS) {
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int c = 0; c < n_chunks; ++c) {
+        const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(mine, c) + 4 * i);
+        o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
+      }
+      *reinterpret_cast<float4*>(out_rows + 4 * i) = o;
+    }
+  }
+  cluster.sync();                                          // (the sums are read by the first CTA until here)
+}
+
 // What a CTA's last step needs, parked in shared memory at its start so that it does not occupy
 // registers across the tile loop.
 struct EpiInfo {
@@ -614,8 +636,7 @@ struct EpiInfo {
 // to aux[(query head) * aux_stride + stripe row] for stripe rows < t_eff (the K kernel of the
 // two-stage interface; V is not read).  MODE_WEIGHTS: the softmax weights are given in
 // aux[(query head) * aux_stride + stripe row]; only sum_t w.V is computed (the V kernel of the
-// two-stage interface; K is not read), records carry m = 0 and l = 1 in chunk 0 so that the
-// combine kernel adds the chunks up.
+// two-stage interface; K is not read); a unit's chunks are a cluster of CTAs (cluster_sum).
 // MODE_ATTN_TAIL: MODE_ATTN over the packed zones plus, in the same softmax, the uncompressed tail
 // of decode-appended tokens (a fifth tile phase of plain 16-bit K and V rows) and the token being
 // decoded, with the rotary embedding of the query rows and of the new key row applied on the way
@@ -837,8 +858,11 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
                     : nullptr;
   const int64_t rec_stride = (int64_t)n_chunks * RDKV_PARTIAL_STRIDE;
   const bool direct = (n_chunks == 1 && out != nullptr);
+  // (MODE_WEIGHTS in chunks: the chunk's sums stay in shared memory, behind the area the warps merge in)
+  float* const cluster_part = reinterpret_cast<float*>(smem_raw) + FW * GH * D;
+  const bool in_cluster = MODE == MODE_WEIGHTS && n_chunks > 1;
   if (tid == 0) {
-    s_epi.out_rows = out != nullptr ? out + ((int64_t)view_idx * H_q + hq0) * D : nullptr;
+    s_epi.out_rows = in_cluster ? cluster_part : out != nullptr ? out + ((int64_t)view_idx * H_q + hq0) * D : nullptr;
     s_epi.rec0 = rec0; s_epi.rec_stride = rec_stride; s_epi.row0 = (int64_t)view_idx * H_q + hq0;
     s_epi.how = MODE == MODE_WEIGHTS ? 2 : direct ? 1 : 0;
     s_epi.gcnt = gcnt; s_epi.n_chunks = n_chunks; s_epi.unit_y = unit_y;
@@ -1088,6 +1112,11 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
   if (total_tiles < 0 || (total_tiles == 0 && !seeded)) {  // nothing live here: empty records
     if (total_tiles < 0 && tid == 0 && status != nullptr) atomicOr(status, 2);
     if (MODE == MODE_SCORES) return;
+    if (in_cluster) {
+      for (int i = tid; i < gcnt * D; i += blockDim.x) cluster_part[i] = 0.f;
+      cluster_sum(cluster_part, gcnt, n_chunks, out + ((int64_t)view_idx * H_q + hq0) * D);
+      return;
+    }
     if (direct) {
       for (int i = tid; i < gcnt * D; i += blockDim.x) out[((int64_t)view_idx * H_q + hq0) * D + i] = 0.f;
     } else {
@@ -1324,6 +1353,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
   final_merge<false>(red, &s_ml[0][0][0], ep.gcnt, ep.how, ep.out_rows, ep.rec0, ep.rec_stride);
   if (ATTN && ep.n_chunks > 1 && unit_ctr != nullptr)
     chunk_merge<false>(partials, unit_ctr + ep.unit_y, ep.n_chunks, ep.gcnt, ep.row0, out, merged);
+  if (MODE == MODE_WEIGHTS && ep.n_chunks > 1) cluster_sum(cluster_part, ep.gcnt, ep.n_chunks, out + ep.row0 * D);
 }
 
 
@@ -1888,10 +1918,23 @@ static int launch_fused(const rdkv_layer_view* views, int n_views, const void* q
   if (tail != nullptr) ta = *tail;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
-  kernel<<<(unsigned)items, CTA_THREADS, smem, (cudaStream_t)stream>>>(
-      views, q, q_dtype, H_q, g, chunk_rows, n_chunks, n_whole, stage_bytes, partials, out, status, aux, aux_stride, t_eff,
-      reinterpret_cast<const UnitRec*>(unit_recs), reinterpret_cast<const KSlotRec*>(kslots), nkb_max, unit_ctr, merged,
-      row_begin, row_end, part, parts, ta);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)items);
+  cfg.blockDim = dim3(CTA_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[1];
+  if (MODE == MODE_WEIGHTS && n_chunks > 1) {                // the chunks of a unit: one cluster
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = n_chunks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  e = cudaLaunchKernelEx(&cfg, kernel, views, q, q_dtype, H_q, g, chunk_rows, n_chunks, n_whole, stage_bytes,
+                         partials, out, status, aux, aux_stride, t_eff, reinterpret_cast<const UnitRec*>(unit_recs),
+                         reinterpret_cast<const KSlotRec*>(kslots), nkb_max, unit_ctr, merged, row_begin, row_end, part, parts,
+                         (const TailArgs)ta);
+  if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
   return launch_status();
 }
 
@@ -2170,6 +2213,16 @@ extern "C" int rdkv_decode_weighted_sum(const rdkv_layer_view* views, int n_view
   if (n_views > 1) return RDKV_ERR_BAD_ARG;                 // one weight matrix per call
   const int rc = check_fused_args(views, n_views, weights, RDKV_F32, H_q, H_kv, k_row_bytes_max);
   if (rc != RDKV_OK || n_views == 0) return rc;
-  return launch_fused<MODE_WEIGHTS>(views, n_views, weights, RDKV_F32, H_q, H_kv, unit_rows, 1, k_row_bytes_max,
+  // One view has H_kv units: a CTA each left 140 SMs idle (8 heads x 1792 rows: 30 us).  A unit's rows are cut
+  // into up to 8 chunks (a portable cluster) of at least 128 rows while the chunks fit the chip.
+  int dev = 0, sms = 0, chunks = 1;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    g_last_cuda_error = (int)cudaGetLastError();
+    return RDKV_ERR_LAUNCH;
+  }
+  const int64_t units = (int64_t)n_views * H_kv * ((H_q / H_kv + GH - 1) / GH);
+  while (chunks < 8 && unit_rows / (2 * chunks) >= 128 && units * 2 * chunks <= 2 * sms) chunks *= 2;
+  const int chunk_rows = ((unit_rows + chunks - 1) / chunks + 63) & ~63;
+  return launch_fused<MODE_WEIGHTS>(views, n_views, weights, RDKV_F32, H_q, H_kv, chunk_rows, chunks, k_row_bytes_max,
                                     nullptr, out, status, const_cast<float*>(weights), weights_row_stride, 0, stream);
 }

@@ -36,7 +36,7 @@ def v_dequant_weighted_sum_dispatch_into(attn_weights_old: torch.Tensor, packed_
     H_q = w.shape[0]
     table = _weights_table(packed_layer, V16, n_v16_per_head, max_T_v, H_q)
     if table is not None and out.is_contiguous() and w.shape[1] >= table.max_t_k:
-        # the weighted-sum half of the fused tensor-core kernel (one CTA per KV head, fixed order)
+        # the weighted-sum half of the fused tensor-core kernel (a cluster of CTAs per KV head, fixed order)
         check(lib().rdkv_decode_weighted_sum(ptr(table.views), 1, H_q, table.H_kv, table.unit_rows,
                                              table.k_row_bytes_max, ptr(w), w.stride(0), ptr(out), ptr(table.status),
                                              stream_ptr(w.device)), "rdkv_decode_weighted_sum")

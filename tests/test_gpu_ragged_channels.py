@@ -47,3 +47,29 @@ def test_k_rows_of_any_width(counts, kept):
     out = packed_decode_attention(q.cuda(), live)
     for i, want in enumerate(wants):
         assert_attn_close(to_np(out[i]), want, f"live view {i}")
+
+
+@pytest.mark.parametrize("rows", [1, 127, 128, 255, 256, 700, 2048])
+@pytest.mark.parametrize("heads,g", [(1, 4), (2, 8), (8, 4), (3, 16)])
+def test_weighted_sum_in_clusters(rows, heads, g):
+    """The V operator cuts a head's rows over a cluster of CTAs: lengths at the edges of the cut, empty
+    chunks, more query heads than one pass takes."""
+    from oracle import ref_attention as RA
+    from rdkv_b200.v_kernel import v_dequant_weighted_sum_dispatch
+    kept = [max(1, rows * (h + 1) // heads) for h in range(heads)]
+    pl, nv = _layer((16, 24, 24), rows + 40, kept, 3, g, H=heads) if heads > 1 else _layer_one(rows, kept, g)
+    w = torch.rand(heads * g, pl.T_eff_k, generator=torch.Generator().manual_seed(1)) / rows
+    got = v_dequant_weighted_sum_dispatch(w.cuda(), pl, V16=None if nv is None else nv[0], n_v16_per_head=pl.n_v16_per_head,
+                                          max_T_v=pl.T_eff)
+    assert_attn_close(to_np(got), RA.v_weighted_sum(w.numpy(), layer_to_np(pl), to_np(nv)), f"{rows} rows")
+    again = v_dequant_weighted_sum_dispatch(w.cuda(), pl, V16=None if nv is None else nv[0], n_v16_per_head=pl.n_v16_per_head,
+                                            max_T_v=pl.T_eff)
+    assert torch.equal(got, again), "the order of the sums is fixed"
+
+
+def _layer_one(rows, kept, g):
+    from rdkv_b200 import synth
+    from rdkv_b200.packing import pack_kv
+    K, V = synth.make_kv(1, rows + 40, seed=3)
+    vb = synth.make_v_bits(1, rows + 40, kept[0], seed=3)
+    return pack_kv(K.cuda(), V.cuda(), vb.cuda(), synth.make_k_bits(1, seed=3).cuda(), g)
