@@ -433,7 +433,7 @@ int rdkv_tail_attn_partial(const void* q, int q_dtype, int64_t n_views, int H_q,
  * W window positions x 128 (q_head_stride, q_row_stride in elements; KV head bh owns query heads
  * bh*g .. bh*g+g-1), k: [BH][T][128]; dtype RDKV_F16 or RDKV_BF16 for both; causal: window position
  * w sees keys <= T-W+w.  g*W <= 256.  scratch: rdkv_obs_scratch_words(BH, g, W, T) 4-byte words.
- * Three launches (row statistics, reduction, token sums); the keys are read twice.  The products run
+ * Three launches (row statistics, reduction, token sums), programmatic dependents of each other; the keys are read twice.  The products run
  * on the tensor cores (tcgen05.mma into tensor memory); the operands are staged by tiled TMA when the
  * base addresses are 16-byte aligned, the strides multiples of 8 elements and W a multiple of 8, by
  * plain loads otherwise (same results).  The device code waits on mbarriers with a limit: the last
@@ -443,6 +443,11 @@ int64_t rdkv_obs_scratch_words(int BH, int g, int W, int T);
 int rdkv_obs_scores(const void* q_obs, const void* k, int dtype, int64_t q_head_stride, int64_t q_row_stride,
                     int64_t k_head_stride, int64_t k_row_stride, int BH, int g, int W, int T, int causal,
                     float* scratch, float* layer_token, float* layer_channel, void* stream);
+/* The same with every token score divided by the number of window positions that see the key (the
+ * reference's correct_norm, obkv_fast.py:1342-1344, 1461). */
+int rdkv_obs_scores_normalised(const void* q_obs, const void* k, int dtype, int64_t q_head_stride, int64_t q_row_stride,
+                               int64_t k_head_stride, int64_t k_row_stride, int BH, int g, int W, int T, int causal,
+                               float* scratch, float* layer_token, float* layer_channel, void* stream);
 int rdkv_score_chunks(int T);
 int64_t rdkv_score_scratch_words(int BH, int T, int D);
 int rdkv_score_layer(const void* aw, int aw_dtype, const void* q, int q_dtype, const void* k, int k_dtype,

@@ -136,6 +136,7 @@ _PROTOTYPES = {
                      _i, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _p], _i),
     "rdkv_obs_scratch_words": ([_i, _i, _i, _i], _i64),
     "rdkv_obs_scores": ([_p, _p, _i, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _i, _p, _p, _p, _p], _i),
+    "rdkv_obs_scores_normalised": ([_p, _p, _i, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _i, _p, _p, _p, _p], _i),
     "rdkv_score_chunks": ([_i], _i),
     "rdkv_score_scratch_words": ([_i, _i, _i], _i64),
     "rdkv_score_layer": ([_p, _i, _p, _i, _p, _i, _i64, _i64, _i, _i, _i, _i, _p, _p, _p, _p], _i),

@@ -209,8 +209,17 @@ struct ObsArgs {
   float* stats;        // [BH][R][2] maxima and sums over all keys
   float* token;        // [BH][T]
   float* channel;      // [BH][128]
+  int normalise;       // token scores over the number of window positions that see the key
+  int* cta_status;     // [BH][P] the first pass's CTAs; merged into `status` by obs_reduce_kernel
   int* status;         // bit 0: operands did not arrive, bit 1: products did not complete
 };
+
+// The three kernels of a call are launched as programmatic dependents of each other: the next one's CTAs
+// start, set up and fetch their first operands while the last CTAs of the one before finish, and wait here
+// before they read its results.  (8 heads x 32768 keys x 128 query rows: 74.9 us in eight launches, with the
+// status word's memset and the normalisation as element-wise ones, 58.1 us in these three.)
+__device__ __forceinline__ void obs_wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void obs_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // The channel score of KV head bh = mean(q^2) * mean_t(k^2), by one CTA of OBS_THREADS threads:
 // threads (half, channel) sum every other row / CTA sum, the halves are added at the end.  Runs as
@@ -247,6 +256,7 @@ obs_stream_kernel(const ObsArgs A, const __grid_constant__ CUtensorMap tm_q, con
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (PASS == 1 && (int)blockIdx.y < A.extra_rows) {        // the grid's first rows: one CTA per head for the channel scores
     const int head = blockIdx.y * gridDim.x + blockIdx.x;
+    obs_wait_for_previous();
     if (head < A.BH) obs_channel_score<BF16>(A, head, s_col);
     return;
   }
@@ -263,6 +273,7 @@ obs_stream_kernel(const ObsArgs A, const __grid_constant__ CUtensorMap tm_q, con
   const uint32_t tmem_cols = 2 * acc_cols;
   const bool k_al = (A.k_row_stride & 7) == 0 && (A.k_head_stride & 7) == 0 && (reinterpret_cast<uintptr_t>(A.k) & 15) == 0;
   const uint16_t* k_head = A.k + bh * A.k_head_stride;
+  int trouble = 0;                                           // thread 0: what goes into the status
 
   if (tid == 0) {
 #pragma unroll
@@ -287,16 +298,6 @@ obs_stream_kernel(const ObsArgs A, const __grid_constant__ CUtensorMap tm_q, con
       const int t0 = (cx + n * P) * OBS_KEYS;
       obs_stage(s_k + n * OBS_BLOCK, OBS_PANEL, 0, k_head + (int64_t)t0 * A.k_row_stride, A.k_row_stride, OBS_KEYS,
                 min(OBS_KEYS, T - t0), k_al);
-    }
-  if (PASS == 1)
-    for (int r = tid; r < OBS_MAX_ROWS; r += OBS_THREADS) {
-      float2 ci = make_float2(0.f, 0.f);
-      if (r < R) {
-        const float2 ml = *reinterpret_cast<const float2*>(A.stats + ((int64_t)bh * R + r) * 2);
-        ci = make_float2(ml.x * OBS_LOG2E, __frcp_rn(ml.y));
-      }
-      s_ci[r] = ci;
-      s_lim[r] = A.causal ? T - A.W + (r % A.W) : T - 1;
     }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the plain stores above, as the tensor cores will see them
   obs_fence_before();
@@ -327,7 +328,7 @@ obs_stream_kernel(const ObsArgs A, const __grid_constant__ CUtensorMap tm_q, con
   auto issue_tile = [&](int n) {
     const int b = n & 1;
     if (!obs_bar_wait(bar0 + 8 * b, (uint32_t)(n >> 1) & 1u)) {
-      atomicOr(A.status, 1);
+      trouble |= 1;
       obs_bar_wait(bar0 + 8 * b, (uint32_t)(n >> 1) & 1u);   // (one more bounded wait for the copies in flight)
       obs_bar_arrive(bar0 + 8 * (2 + b));
       return;
@@ -357,6 +358,18 @@ obs_stream_kernel(const ObsArgs A, const __grid_constant__ CUtensorMap tm_q, con
     if (n_my > 1) load_tile(1, false);
     issue_tile(0);
   }
+  if (PASS == 1) {                                           // (read by the tile loop behind its first barrier)
+    obs_wait_for_previous();
+    for (int r = tid; r < OBS_MAX_ROWS; r += OBS_THREADS) {
+      float2 ci = make_float2(0.f, 0.f);
+      if (r < R) {
+        const float2 ml = *reinterpret_cast<const float2*>(A.stats + ((int64_t)bh * R + r) * 2);
+        ci = make_float2(ml.x * OBS_LOG2E, __frcp_rn(ml.y));
+      }
+      s_ci[r] = ci;
+      s_lim[r] = A.causal ? T - A.W + (r % A.W) : T - 1;
+    }
+  }
 
   const int q4 = warp & 3, half = warp >> 2;
   // PASS 0: a thread's rows (one per row block), their running statistics over this half of the keys; its share of k^2
@@ -367,7 +380,7 @@ obs_stream_kernel(const ObsArgs A, const __grid_constant__ CUtensorMap tm_q, con
 #pragma unroll 1
   for (int n = 0; n < n_my; ++n) {
     const int b = n & 1, tile = cx + n * P, t0 = tile * OBS_KEYS, n_keys = min(OBS_KEYS, T - t0);
-    if (tid == 0 && !obs_bar_wait(bar0 + 8 * (2 + b), (uint32_t)(n >> 1) & 1u)) atomicOr(A.status, 2);
+    if (tid == 0 && !obs_bar_wait(bar0 + 8 * (2 + b), (uint32_t)(n >> 1) & 1u)) trouble |= 2;
     __syncthreads();                                         // tile n's products are complete (and everybody is done with tile n-1)
     obs_fence_after();
     if (tid == 0) {
@@ -485,11 +498,17 @@ obs_stream_kernel(const ObsArgs A, const __grid_constant__ CUtensorMap tm_q, con
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       if (tid == 0) load_tile(n + 2, false);                 // (the arrival that stands for the copies; the products are issued after the next CTA barrier)
     }
-    if (PASS == 1 && tid < n_keys)                           // (the reference's aw.sum(...) is in aw's type)
-      A.token[(int64_t)bh * T + t0 + tid] = obs_round<BF16>(s_col[tid] + s_col[OBS_KEYS + tid]);
+    if (PASS == 1 && tid < n_keys) {                         // (the reference's aw.sum(...) is in aw's type)
+      const int t = t0 + tid, seen = A.causal ? min(A.W, T - t) : A.W;
+      const float x = obs_round<BF16>(s_col[tid] + s_col[OBS_KEYS + tid]);
+      A.token[(int64_t)bh * T + t] = A.normalise ? __fdiv_rn(x, (float)seen) : x;
+    }
   }
 
+  if (PASS == 1 && trouble != 0) atomicOr(A.status, trouble);
   if (PASS == 0) {
+    obs_let_next_start();
+    if (tid == 0) A.cta_status[bh * P + cx] = trouble;
 #pragma unroll
     for (int mb = 0; mb < 2; ++mb) {
       const int row = mb * OBS_ROWS + q4 * 32 + lane;
@@ -530,6 +549,14 @@ obs_reduce_kernel(ObsArgs A) {
   __shared__ float2 s_ml[OBS_RED_SLICES][OBS_RED_ROWS];
   const int bh = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int R = A.g * A.W, n_parts = 2 * A.P;
+  obs_let_next_start();
+  obs_wait_for_previous();
+  if (blockIdx.x == 0 && bh == 0) {                          // the first pass's status words
+    int any = 0;
+    for (int i = tid; i < A.BH * A.P; i += OBS_RED_THREADS) any |= A.cta_status[i];
+    any = __syncthreads_or(any & 1) | __syncthreads_or(any & 2) << 1;
+    if (tid == 0) *A.status = any;
+  }
   const int r = tid & (OBS_RED_ROWS - 1), slice = tid / OBS_RED_ROWS;
   const int row = blockIdx.x * OBS_RED_ROWS + r;
   float M = -INFINITY, L = 0.f;
@@ -610,13 +637,12 @@ using namespace rdkv;
 extern "C" int64_t rdkv_obs_scratch_words(int BH, int g, int W, int T) {
   if (BH < 0 || g <= 0 || W <= 0 || T <= 0) return 0;
   const int64_t n_tiles = (T + OBS_KEYS - 1) / OBS_KEYS, R = (int64_t)g * W;   // (sized for one CTA per tile; fewer run)
-  return BH * (2 * n_tiles * R * 2 + n_tiles * 128 + R * 2) + 1;
+  return BH * (2 * n_tiles * R * 2 + n_tiles * 128 + R * 2 + n_tiles) + 1;
 }
 
-extern "C" int rdkv_obs_scores(const void* q_obs, const void* k, int dtype, int64_t q_head_stride,
-                               int64_t q_row_stride, int64_t k_head_stride, int64_t k_row_stride, int BH, int g,
-                               int W, int T, int causal, float* scratch, float* layer_token, float* layer_channel,
-                               void* stream) {
+static int obs_scores(const void* q_obs, const void* k, int dtype, int64_t q_head_stride, int64_t q_row_stride,
+                      int64_t k_head_stride, int64_t k_row_stride, int BH, int g, int W, int T, int causal, int normalise,
+                      float* scratch, float* layer_token, float* layer_channel, void* stream) {
   if (q_obs == nullptr || k == nullptr || scratch == nullptr || layer_token == nullptr || layer_channel == nullptr)
     return RDKV_ERR_BAD_ARG;
   if (dtype != RDKV_F16 && dtype != RDKV_BF16) return RDKV_ERR_BAD_ARG;
@@ -632,7 +658,7 @@ extern "C" int rdkv_obs_scores(const void* q_obs, const void* k, int dtype, int6
   ObsArgs A;
   A.q = reinterpret_cast<const uint16_t*>(q_obs); A.k = reinterpret_cast<const uint16_t*>(k);
   A.q_head_stride = q_head_stride; A.q_row_stride = q_row_stride; A.k_head_stride = k_head_stride; A.k_row_stride = k_row_stride;
-  A.g = g; A.W = W; A.T = T; A.causal = causal ? 1 : 0; A.n_tiles = (T + OBS_KEYS - 1) / OBS_KEYS;
+  A.g = g; A.W = W; A.T = T; A.causal = causal ? 1 : 0; A.normalise = normalise; A.n_tiles = (T + OBS_KEYS - 1) / OBS_KEYS;
   const int64_t R = (int64_t)g * W;
   const int MB = (int)((R + OBS_ROWS - 1) / OBS_ROWS);
   // CTAs per head: the resident CTAs (two per SM with one row block, one with two) shared out over the heads
@@ -643,7 +669,8 @@ extern "C" int rdkv_obs_scores(const void* q_obs, const void* k, int dtype, int6
   A.part = scratch;
   A.ksq = A.part + (int64_t)BH * 2 * A.n_tiles * R * 2;
   A.stats = A.ksq + (int64_t)BH * A.n_tiles * 128;
-  A.status = reinterpret_cast<int*>(A.stats + (int64_t)BH * R * 2);
+  A.cta_status = reinterpret_cast<int*>(A.stats + (int64_t)BH * R * 2);
+  A.status = A.cta_status + (int64_t)BH * A.n_tiles;
   A.token = layer_token; A.channel = layer_channel;
   // the operands come by TMA when their layout can be mapped; a head's W query rows are one box,
   // which must start on a group of 8 rows
@@ -653,8 +680,6 @@ extern "C" int rdkv_obs_scores(const void* q_obs, const void* k, int dtype, int6
   A.tma_q = (W % 8 == 0 && obs_map(&tm_q, q_obs, bf, q_head_stride, q_row_stride, (int64_t)BH * g, W, W)) ? 1 : 0;
   const size_t smem = 1024 + (size_t)(2 + MB) * OBS_BLOCK;   // (the base is rounded up to 1024 bytes in the kernel)
   cudaStream_t st = (cudaStream_t)stream;
-  e = cudaMemsetAsync(A.status, 0, sizeof(int), st);
-  if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
   auto launch = [&](auto kern_stats, auto kern_token) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern_stats, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern_token, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -662,12 +687,40 @@ extern "C" int rdkv_obs_scores(const void* q_obs, const void* k, int dtype, int6
     kern_stats<<<dim3(A.P, BH), OBS_THREADS, smem, st>>>(A, tm_q, tm_k);
     int rc = launch_status();
     if (rc != RDKV_OK) return rc;
-    obs_reduce_kernel<<<dim3((unsigned)((R + OBS_RED_ROWS - 1) / OBS_RED_ROWS), BH), OBS_RED_THREADS, 0, st>>>(A);
-    rc = launch_status();
-    if (rc != RDKV_OK) return rc;
-    kern_token<<<dim3(A.P, BH + A.extra_rows), OBS_THREADS, smem, st>>>(A, tm_q, tm_k);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)((R + OBS_RED_ROWS - 1) / OBS_RED_ROWS), BH);
+    cfg.blockDim = dim3(OBS_RED_THREADS);
+    e = cudaLaunchKernelEx(&cfg, obs_reduce_kernel, A);
+    if (e == cudaSuccess) {
+      cfg.gridDim = dim3(A.P, BH + A.extra_rows);
+      cfg.blockDim = dim3(OBS_THREADS);
+      cfg.dynamicSmemBytes = smem;
+      e = cudaLaunchKernelEx(&cfg, kern_token, (const ObsArgs)A, tm_q, tm_k);
+    }
+    if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
     return launch_status();
   };
   if (bf) return launch(obs_stream_kernel<true, 0>, obs_stream_kernel<true, 1>);
   return launch(obs_stream_kernel<false, 0>, obs_stream_kernel<false, 1>);
+}
+
+extern "C" int rdkv_obs_scores(const void* q_obs, const void* k, int dtype, int64_t q_head_stride, int64_t q_row_stride,
+                               int64_t k_head_stride, int64_t k_row_stride, int BH, int g, int W, int T, int causal,
+                               float* scratch, float* layer_token, float* layer_channel, void* stream) {
+  return obs_scores(q_obs, k, dtype, q_head_stride, q_row_stride, k_head_stride, k_row_stride, BH, g, W, T, causal, 0, scratch,
+                    layer_token, layer_channel, stream);
+}
+
+extern "C" int rdkv_obs_scores_normalised(const void* q_obs, const void* k, int dtype, int64_t q_head_stride,
+                                          int64_t q_row_stride, int64_t k_head_stride, int64_t k_row_stride, int BH, int g,
+                                          int W, int T, int causal, float* scratch, float* layer_token,
+                                          float* layer_channel, void* stream) {
+  return obs_scores(q_obs, k, dtype, q_head_stride, q_row_stride, k_head_stride, k_row_stride, BH, g, W, T, causal, 1, scratch,
+                    layer_token, layer_channel, stream);
 }

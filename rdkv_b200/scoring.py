@@ -74,19 +74,15 @@ def obs_window_scores(q_obs: Tensor, k: Tensor, *, causal: bool = True, normalis
     token = torch.empty((B, H, T), dtype=torch.float32, device=dev)
     channel = torch.empty((B, H, D), dtype=torch.float32, device=dev)
     scratch = torch.empty(lib().rdkv_obs_scratch_words(B * H, g, W, T), dtype=torch.float32, device=dev)
-    check(lib().rdkv_obs_scores(ptr(q_obs), ptr(k), q_dtype_tag(q_obs), q_obs.stride(1), q_obs.stride(2), k.stride(1),
-                                k.stride(2), B * H, g, W, T, 1 if causal else 0, ptr(scratch), ptr(token), ptr(channel),
-                                stream_ptr(dev)), "rdkv_obs_scores")
+    fn = lib().rdkv_obs_scores_normalised if normalise else lib().rdkv_obs_scores
+    check(fn(ptr(q_obs), ptr(k), q_dtype_tag(q_obs), q_obs.stride(1), q_obs.stride(2), k.stride(1),
+             k.stride(2), B * H, g, W, T, 1 if causal else 0, ptr(scratch), ptr(token), ptr(channel),
+             stream_ptr(dev)), "rdkv_obs_scores")
     if check_status:
         status = int(scratch[-1:].view(torch.int32).item())    # (the last scratch word)
         if status != 0:
             raise RuntimeError(f"rdkv_obs_scores: a device-side wait ran out (status {status}: 1 = operands, "
                                f"2 = products); the scores are invalid")
-    if normalise:
-        norm = torch.full((T,), float(W), dtype=torch.float32, device=dev)
-        if causal:
-            norm[T - W:] = torch.arange(W, 0, -1, dtype=torch.float32, device=dev)
-        token = token / norm
     return token, channel
 
 

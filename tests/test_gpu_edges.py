@@ -149,3 +149,20 @@ def test_unpack_rows(rows, mix):
         assert np.array_equal(to_np(k).view(np.uint16), want_k.view(np.uint16))
         assert np.array_equal(to_np(v).view(np.uint16), want_v.view(np.uint16))
         assert torch.equal(unpack_k_mixed(pl, 128), k)
+
+
+@pytest.mark.parametrize("tokens,window,g", [(33, 32, 4), (128, 8, 4), (129, 16, 8), (1000, 32, 8), (5000, 5, 3)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_normalised_window_scores(tokens, window, g, causal):
+    """The division by the window positions that see a key, inside the second pass: the fp32 quotient of the
+    plain call's scores, for tiles of 128 keys that end inside the window and windows staged by plain loads."""
+    from rdkv_b200.scoring import obs_window_scores
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    q = torch.randn(1, 2 * g, window, 128, generator=gen, device="cuda").half()
+    k = torch.randn(1, 2, tokens, 128, generator=gen, device="cuda").half()
+    plain, channel = obs_window_scores(q, k, causal=causal, check_status=True)
+    token, channel_n = obs_window_scores(q, k, causal=causal, normalise=True, check_status=True)
+    seen = torch.full((tokens,), float(window), device="cuda")
+    if causal:
+        seen[tokens - window:] = torch.arange(window, 0, -1, device="cuda", dtype=torch.float32)
+    assert torch.equal(token, plain / seen) and torch.equal(channel, channel_n)
