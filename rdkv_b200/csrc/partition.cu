@@ -12,17 +12,19 @@ namespace rdkv {
 // Bound by the reads of the maps (8 bytes an element as the allocator returns them) and, for few rows, by
 // latency.  A row is cut into runs for a cluster of CTAs, a CTA's run into runs for its warps, a warp's run
 // into tiles of 256 elements: eight neighbouring ones per lane (vector loads where they are aligned).  A lane
-// classifies its eight elements once and keeps what the second step needs as one register per tile (four
-// bits an element: kept, class bit 0, class bit 1, compressed); that step writes every kept element to
-// its place and does not read the map again.  Places: counts per lane, scanned over the warp tile by tile,
+// classifies its eight elements once and keeps what the second step needs as one word per tile in shared
+// memory (four bits an element: kept, class bit 0, class bit 1, compressed); that step writes every kept
+// element to its place and does not read the map again.  Places: counts per lane, scanned over the warp tile by tile,
 // over the warps once, over the cluster once (distributed shared memory).
-// One CTA per row with one run per thread (the previous form) read 64-bit maps 1 KB apart within a warp
-// and left most SMs idle.  64-bit maps, kernel time: 32 rows x 131072 813 us (four launches of 8 rows) -> 26 us,
-// 256 x 32768 55 -> 38 us, 8 x 32768 28 -> 10 us; 16-bit maps, 256 x 32768: 23 -> 32 us (every tile is turned into
-// flags first), 32 x 131072: 770 -> 23 us.
+// One CTA per row with one run per thread (an earlier form) read 64-bit maps 1 KB apart within a warp
+// and left most SMs idle.  64-bit maps, kernel time: 32 rows x 131072 813 us (four launches of 8 rows) -> 18 us,
+// 256 x 32768 55 -> 29 us, 8 x 32768 28 -> 8 us; 16-bit maps, 256 x 32768: 23 -> 28 us (every tile is turned into
+// flags first), 32 x 131072: 770 -> 17 us.
+// (Two CTAs per SM, classes in registers and the loops unrolled by the tiles: 26, 38, 10, 32 and 23 us, 28 us for
+// four layers of 131072 rows in one launch, now 21; most of a warp's time went into instruction fetches.)
 constexpr int PT_THREADS = 512;
 constexpr int PT_WARPS = PT_THREADS / 32;
-constexpr int PT_TILES = 8;                                 // tiles of a warp whose classes stay in registers
+constexpr int PT_TILES = 8;                                 // tiles of a warp whose classes are kept
 constexpr int PT_MAX_CLUSTER = 8;
 
 struct PartSet {
@@ -103,7 +105,7 @@ __device__ __forceinline__ PartCount part_count(uint32_t f) {
 // fill: entries past a row's kept count become -1.  rank (may be null): for every place in a compressed
 // class the element's number among the row's compressed elements (bits > 0 and not 16) in ascending order.
 template <int ES>
-__device__ __forceinline__ void partition_row(const PartSet& P, int row, int fill, int (*s_warp)[5], int* s_cta) {
+__device__ __forceinline__ void partition_row(const PartSet& P, int row, int fill, uint32_t (*s_flags)[PT_THREADS], int (*s_warp)[5], int* s_cta) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), n_cta = (int)cluster.num_blocks();
@@ -116,8 +118,7 @@ __device__ __forceinline__ void partition_row(const PartSet& P, int row, int fil
   const int64_t lo = min((int64_t)len, (int64_t)(rank * PT_WARPS + warp) * per_warp);
   const int64_t hi = min((int64_t)len, lo + per_warp);
   const int tiles = (int)((hi - lo + 255) >> 8);
-  const bool cached = per_warp <= PT_TILES * 256;           // every tile's classes stay in registers
-  uint32_t flags[PT_TILES];
+  const bool cached = per_warp <= PT_TILES * 256;           // every tile's classes are kept
   PartCount sum = {0u, 0u, 0u};
   auto tile_flags = [&](int t) {
     uint32_t w[8];
@@ -135,16 +136,16 @@ __device__ __forceinline__ void partition_row(const PartSet& P, int row, int fil
     cnt[4] += __reduce_add_sync(0xffffffffu, sum.comp);
     sum = {0u, 0u, 0u};
   };
-  if (cached) {
-#pragma unroll
-    for (int t = 0; t < PT_TILES; ++t) flags[t] = t < tiles ? tile_flags(t) : 0u;
-#pragma unroll
-    for (int t = 0; t < PT_TILES; ++t) note(flags[t]);
-    warp_totals();
-  } else {
-    for (int t = 0; t < tiles; ++t) { note(tile_flags(t)); if ((t & 7) == 7) warp_totals(); }
-    warp_totals();
+  // (both loops over the tiles are kept short: a CTA goes through its code once or twice, and unrolled by
+  //  the tiles it waited for instruction fetches seven cycles per instruction)
+#pragma unroll 1
+  for (int t = 0; t < tiles; ++t) {
+    const uint32_t f = tile_flags(t);
+    if (cached) s_flags[t][tid] = f;
+    note(f);
+    if ((t & 7) == 7) warp_totals();
   }
+  warp_totals();
   if (lane == 0)
 #pragma unroll
     for (int c = 0; c < 5; ++c) s_warp[warp][c] = cnt[c];
@@ -194,30 +195,26 @@ __device__ __forceinline__ void partition_row(const PartSet& P, int row, int fil
     pos[0] += (int)(t01 & 0xFFFFu); pos[1] += (int)(t01 >> 16); pos[2] += (int)(t23 & 0xFFFFu); pos[3] += (int)(t23 >> 16);
     comp_at += (int)tcomp;
   };
-  if (cached) {
-#pragma unroll
-    for (int t = 0; t < PT_TILES; ++t)
-      if (t < tiles) place(t, flags[t]);
-  } else {
-    for (int t = 0; t < tiles; ++t) place(t, tile_flags(t));
-  }
+#pragma unroll 1
+  for (int t = 0; t < tiles; ++t) place(t, cached ? s_flags[t][tid] : tile_flags(t));
   if (fill)
     for (int i = kept + rank * PT_THREADS + tid; i < len; i += n_cta * PT_THREADS) orow[i] = -1;
   cluster.sync();                                           // (the totals are read by the other CTAs)
 }
 
-__global__ void __launch_bounds__(PT_THREADS)
+__global__ void __launch_bounds__(PT_THREADS, 3)
 partition_pair_kernel(const __grid_constant__ PartSet A, const __grid_constant__ PartSet B, int fill) {
+  __shared__ uint32_t s_flags[PT_TILES][PT_THREADS];        // a lane's classes of its warp's tiles
   __shared__ int s_warp[PT_WARPS][5];                       // per warp: elements of classes 0..3, compressed elements
   __shared__ int s_cta[5];                                  // the CTA's totals (read by the whole cluster)
   const int r = blockIdx.x / (int)cooperative_groups::this_cluster().num_blocks();
   const PartSet& P = r < A.n_rows ? A : B;
   const int row = r < A.n_rows ? r : r - A.n_rows;
   switch (P.elem_size) {
-    case 1: partition_row<1>(P, row, fill, s_warp, s_cta); break;
-    case 2: partition_row<2>(P, row, fill, s_warp, s_cta); break;
-    case 4: partition_row<4>(P, row, fill, s_warp, s_cta); break;
-    default: partition_row<8>(P, row, fill, s_warp, s_cta); break;
+    case 1: partition_row<1>(P, row, fill, s_flags, s_warp, s_cta); break;
+    case 2: partition_row<2>(P, row, fill, s_flags, s_warp, s_cta); break;
+    case 4: partition_row<4>(P, row, fill, s_flags, s_warp, s_cta); break;
+    default: partition_row<8>(P, row, fill, s_flags, s_warp, s_cta); break;
   }
 }
 
@@ -270,8 +267,8 @@ static int launch_partition(const PartSet& A, const PartSet& B, int fill, cudaSt
     g_last_cuda_error = (int)cudaGetLastError();
     return RDKV_ERR_LAUNCH;
   }
-  // CTAs per row: enough to give every SM one and to keep every tile's classes in registers (eight tiles a
-  // warp), but not less than a tile a warp
+  // CTAs per row: enough to give every SM one and to keep every tile's classes (eight tiles a warp), but not
+  // less than a tile a warp
   const int len = A.len > B.len ? A.len : B.len;
   int cluster = 1;
   while (cluster < PT_MAX_CLUSTER && len > cluster * PT_WARPS * 256 &&
