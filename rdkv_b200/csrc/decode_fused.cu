@@ -6,7 +6,8 @@
 // one tiled TMA box through a tensor map of the view's V tensor, 16 bytes wider than a row, so that
 // the rows land at a pitch at which the P.V operand loads have no bank conflicts — completion
 // counted on an mbarrier.  Warps 0-3 (the compute warps) fold the queries meanwhile and then work through the
-// tiles, 32 rows (two 16-row MMA groups) per warp and step:
+// tiles, 32 rows (two 16-row MMA groups) per warp and step (decode_tile.inc; K rows that are not whole aligned
+// words: decode_tile_wide.inc; tail rows: 16 per warp):
 //   * q.K scores on the tensor cores (mma.sync m16n8k16, rows on M, query heads on N): packed
 //     2/4/8-bit K codes are masked in place into fp16 SUBNORMAL integers (code * 2^-24, exact), so
 //     unpacking is one AND per pair of codes; bit-position factors (4^v, 16) are folded into q*scale;
@@ -69,9 +70,21 @@ constexpr unsigned WAIT_LIMIT = 1u << 22;  // try_wait rounds before a compute w
 constexpr float RESCALE_TH = 8.f;      // log2 slack before the running maximum is moved
 constexpr float M_NONE = -1.0e30f;     // reference maximum of a head that has seen no live score yet (finite: no inf - inf)
 
-// (phase 4 = the uncompressed tail: plain K and V rows of 256 bytes each share the V area of a stage)
 __host__ __device__ constexpr int phase_tile_rows(int p) {
-  return p < 2 ? TILE_MAX : p == 2 ? TILE_MAX / 2 : p == 3 ? TILE_MAX / 4 : TILE_MAX / 8;
+  return p < 2 ? TILE_MAX : p == 2 ? TILE_MAX / 2 : TILE_MAX / 4;
+}
+// Phase 4 = the uncompressed tail: plain K and V rows of 256 bytes each.  A tile has as many rows as fill a
+// whole stage, 16 for each compute warp at most: the K rows from the stage's first byte on, the V rows
+// behind them, with room to clear the V rows up to the next multiple of 16.  (Tiles of 32 rows in the V area
+// gave all their rows to one warp and half a stage to each copy: 16 sequences x 8 heads, 2048 kept and about
+// 390 tail rows, 45.8 -> 34.8 us.)
+__host__ __device__ inline int tail_tile_rows(int stage_bytes) {
+  const int most = 16 * FW;
+  for (int up = most; up > 16; up -= 16) {                 // rows rounded up to a multiple of 16
+    const int n = (stage_bytes - up * 256) / 256;
+    if (n > up - 16) return n < up ? n : up;
+  }
+  return 16;
 }
 __host__ __device__ constexpr int phase_row_bytes(int p) { return p == 0 ? 32 : p == 1 ? 64 : p == 2 ? 128 : 256; }
 // Distance of consecutive V rows in a stage.  A thread of the P.V product reads the same bytes of
@@ -421,14 +434,14 @@ constexpr int PLAN_TILES = 32;         // tiles planned per round (one per stagi
 constexpr int PLAN_TILES_TAIL = 12;    // the same with an uncompressed tail (2.2 KB less: with K rows of up to 49 bytes there is room for three CTAs)
 
 template <int NPH>
-__device__ __forceinline__ TileDesc tile_of(const CtaGeom& G, int idx) {
+__device__ __forceinline__ TileDesc tile_of(const CtaGeom& G, int idx, int tail_tile) {
   TileDesc t;
   int p = 0;
 #pragma unroll
   for (int k = 1; k < NPH; ++k)
     if (idx >= G.first_tile[k]) p = k;
   t.phase = p;
-  const int tr = phase_tile_rows(p);
+  const int tr = NPH > 4 && p == 4 ? tail_tile : phase_tile_rows(p);
   t.row0 = (idx - G.first_tile[p]) * tr;
   t.n = min(tr, G.hi[p] - G.lo[p] - t.row0);
   return t;
@@ -643,10 +656,9 @@ struct EpiInfo {
 // in (TailArgs).  A separate instantiation: the other modes' code is not touched by it.
 constexpr uint32_t K_FEW = 64u;        // (k_spans in decode_state.inc) at most two spans per K segment
 constexpr int MODE_ATTN = 0, MODE_SCORES = 1, MODE_WEIGHTS = 2, MODE_ATTN_TAIL = 3;
-constexpr int TAIL_TILE = TILE_MAX / 8;             // tail rows per tile: K rows and V rows fill the V area together
 constexpr int TAILQ_BYTES = 8 * 32 * 8;             // the queries as fp16 B fragments of the tail's score product
 constexpr int TAIL_EXTRA_BYTES = TAILQ_BYTES + 2 * 128 * 4 + 64;   // + new key row, new value row (fp32), its scores
-static_assert(2 * TAIL_TILE * 256 <= V_STAGE, "a tail tile's K and V rows share the V area");
+static_assert(2 * 16 * 256 <= V_STAGE, "a tail tile of 16 rows fits any stage");
 
 using TailArgs = rdkv_tail_args;
 
@@ -725,6 +737,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
   bool geom_done = false;
   int n_tail = 0;                                          // live rows of the uncompressed tail of this view
   // the tail's share of this CTA, from the rows pn0..pn3 the part has of the four packed phases:
+  const int tail_tile = TAIL ? tail_tile_rows(stage_bytes) : 0;
   // window [lo, hi) in the part's row numbering, first tail row d, tiles
   struct TailGeom { int lo, hi, d, tiles; };
   auto tail_geom = [&](int pn0, int pn1, int pn2, int pn3, int c0, int c1) {
@@ -733,7 +746,7 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
     TailGeom t;
     t.lo = max(lb4, c0); t.hi = max(t.lo, min(lb4 + pn4, c1));
     t.d = ps4 + (t.lo - lb4);
-    t.tiles = (t.hi - t.lo + TAIL_TILE - 1) / TAIL_TILE;
+    t.tiles = (t.hi - t.lo + tail_tile - 1) / tail_tile;
     return t;
   };
   auto tail_row = [&](const void* base, int row) {         // address of a row of this (view, KV head)'s tail buffer
@@ -1149,17 +1162,16 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
       if (slot == 0) {                                     // plan tiles [it, it + PLAN)
         __syncwarp();
         if ((PLAN == 32 || lane < PLAN) && it + lane < total_tiles) {
-          const TileDesc t = tile_of<NPH>(G, it + lane);
+          const TileDesc t = tile_of<NPH>(G, it + lane, tail_tile);
           const int p = t.phase;
           TilePlan& P = s_plan[lane];
           if (TAIL && p == 4) {
-            // tail tile: its V rows at the start of the V area, its K rows behind them; the block
-            // goes to warp (tile number within the tail) % FW
-            P.rg[0] = RangePlan{G.vrow[4] + (int64_t)t.row0 * 256, t.n * 256, (uint32_t)SL.v};
-            P.rg[1] = RangePlan{G.krow_tail + (int64_t)t.row0 * 256, t.n * 256, (uint32_t)(SL.v + TAIL_TILE * 256)};
+            // tail tile: its K rows from the stage's first byte on, its V rows behind them
+            P.rg[0] = RangePlan{G.vrow[4] + (int64_t)t.row0 * 256, t.n * 256, (uint32_t)(tail_tile * 256)};
+            P.rg[1] = RangePlan{G.krow_tail + (int64_t)t.row0 * 256, t.n * 256, 0u};
 #pragma unroll
             for (int k = 2; k < 6; ++k) P.rg[k] = RangePlan{nullptr, 0, 0u};
-            P.info.phase = 4 | ((t.row0 / TAIL_TILE) & (FW - 1)) << 8; P.info.n = t.n;
+            P.info.phase = 4; P.info.n = t.n;
             P.info.offs = 0u; P.info.krow0 = 0;
           } else {
           const unsigned char* a_k2 = G.k2[p] + (int64_t)t.row0 * kd.sub2;
@@ -1251,12 +1263,13 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
         }
       }
       // rows past the tile's end must hold finite fp16 data in the fp16 phase: clear the
-      // rest of the last 32-row block beyond the copied blocks
-      if ((ti.phase & 7) >= 3 && (ti.n & 31)) {
-        const int pitch = phase_pitch(ti.phase & 7);       // (the tail's rows: 256 bytes; fp16 V rows: padded)
+      // rest of the last 32-row block (of the tail's last 16-row group) beyond the copied blocks
+      const bool ti_tail = TAIL && (ti.phase & 7) == 4;
+      if ((ti.phase & 7) >= 3 && (ti.n & (ti_tail ? 15 : 31))) {
+        const int pitch = ti_tail ? 256 : phase_pitch(3);
         const int first = ti.n * pitch;
-        const int last = min(((ti.n + 31) & ~31) * pitch, V_STAGE);
-        unsigned char* sv = smem_raw + (size_t)stage * stage_bytes + SL.v;
+        const int last = ti_tail ? ((ti.n + 15) & ~15) * 256 : min(((ti.n + 31) & ~31) * pitch, V_STAGE);
+        unsigned char* sv = smem_raw + (size_t)stage * stage_bytes + (ti_tail ? tail_tile * 256 : SL.v);
         for (int i = first + 4 * lane; i < last; i += 4 * 32) *reinterpret_cast<uint32_t*>(sv + i) = 0u;
       }
       if (lane == 0) s_tile[stage] = ti;
@@ -1310,9 +1323,9 @@ decode_fused_kernel(const rdkv_layer_view* __restrict__ views, const void* __res
     // this warp takes the tile's 32-row blocks pb, pb+FW, ... (two 16-row MMA groups each, worked on
     // together so that the two dependency chains overlap); the start rotates from tile to tile so
     // that short tiles (fewer blocks than warps) do not always land on the same warps
-    const int nblocks = (t.n + 31) >> 5;
-    const int pb = (TAIL && p == 4) ? (warp + FW - ((t.phase >> 8) & (FW - 1))) % FW
-                                    : (warp + FW - (it * (TILE_MAX / 128)) % FW) % FW;
+    // (a tail tile: one 16-row group per warp)
+    const int nblocks = (TAIL && p == 4) ? (t.n + 15) >> 4 : (t.n + 31) >> 5;
+    const int pb = (warp + FW - (it * (TILE_MAX / 128)) % FW) % FW;
 
     if constexpr (WIDE) {
 #include "decode_tile_wide.inc"
@@ -1549,7 +1562,7 @@ decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, i
         if (slot == 0) {                                   // plan tiles [it, it + 32)
           __syncwarp();
           if (it + lane < total) {
-            const TileDesc t = tile_of<4>(G, it + lane);
+            const TileDesc t = tile_of<4>(G, it + lane, 0);
             const int tp = t.phase;
             TilePlan& P = s_plan[lane];
             const unsigned char* a_k2 = G.k2[tp] + (int64_t)t.row0 * kd.sub2;
@@ -1732,6 +1745,7 @@ decode_persist_kernel(const void* __restrict__ q, int q_dtype, int H_q, int g, i
   float tref_e = 0.f, tref_o = 0.f;
   const uint32_t qt_lane = 0u;
   const bool tail_bf = false;
+  constexpr int tail_tile = 0;
 #include "decode_state.inc"
 #pragma unroll 1
       for (int it = 0; it < n_it; ++it) {

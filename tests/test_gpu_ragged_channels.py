@@ -49,6 +49,34 @@ def test_k_rows_of_any_width(counts, kept):
         assert_attn_close(to_np(out[i]), want, f"live view {i}")
 
 
+@pytest.mark.parametrize("counts", [(16, 24, 24), (23, 31, 35), (3, 17, 100), (1, 0, 0)])
+@pytest.mark.parametrize("tails", [(1, 15), (16, 17), (31, 33), (47, 49), (63, 64), (65, 127), (129, 500)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_tail_tiles(counts, tails, dtype):
+    """Tail lengths at the edges of a warp's 16 rows and of a tile, for stages of several sizes, whole units
+    and chunks; rows behind the live ones are not numbers and must not show."""
+    from oracle import ref_attention as RA
+    from rdkv_b200 import synth
+    from rdkv_b200.decode import DecodeTable, packed_decode_attention
+    g, H, cap = 4, 2, 512
+    layers = [_layer(counts, 400, [201, 77], 11, g), _layer(counts, 401, [5, 300], 12, g)]
+    gen = torch.Generator().manual_seed(sum(tails))
+    q = synth.make_q(H * g, seed=6, batch=2, dtype=dtype)
+    new = torch.randn(2, 2, H, cap, 128, generator=gen).to(dtype)            # K, V
+    wants = [RA.decode_attention(q[i].float().numpy(), layer_to_np(pl), to_np(nv), new[0, i, :, :tails[i]].float().numpy(),
+                                 new[1, i, :, :tails[i]].float().numpy())[0] for i, (pl, nv) in enumerate(layers)]
+    for i in range(2):
+        new[:, i, :, tails[i]:] = float("nan")
+    new = new.cuda()
+    n_new = torch.tensor(tails, dtype=torch.int32, device="cuda")
+    for n_chunks in (None, 3):
+        table = DecodeTable([p for p, _ in layers], [n for _, n in layers], H * g, n_chunks=n_chunks)
+        out = packed_decode_attention(q.cuda(), table, new_k=new[0], new_v=new[1], n_new=n_new)
+        table.check_status()
+        for i, want in enumerate(wants):
+            assert_attn_close(to_np(out[i]), want, f"view {i}, chunks {n_chunks}")
+
+
 @pytest.mark.parametrize("rows", [1, 127, 128, 255, 256, 700, 2048])
 @pytest.mark.parametrize("heads,g", [(1, 4), (2, 8), (8, 4), (3, 16)])
 def test_weighted_sum_in_clusters(rows, heads, g):
