@@ -326,14 +326,21 @@ knapsack_bucket_kernel(const float* __restrict__ scores, int64_t row_stride, int
 
 // Short rows (K channels, small blocks): a warp per row, PER scores per lane in registers.  A sweep is PER
 // evaluations a lane and one warp-wide addition, without a barrier.
+// ALONE: up to 16 rows (the heads of a layer) in one CTA, which replays the batch-wide exit of the doubling
+// loop on the seeds it has in shared memory, so that no second launch has to look for rows to do again (one
+// layer selected and packed: 286 -> 280 us; four blocks of 64 tokens: 954 -> 920 us).  More rows than one CTA
+// has warps would not share its memory, and their second launch is a small part of their call.
 constexpr int KW_WARPS = 4;
-template <int PER>
-__global__ void __launch_bounds__(KW_WARPS * 32)
+constexpr int KW_ALONE = 16;
+template <int PER, bool ALONE>
+__global__ void __launch_bounds__((ALONE ? KW_ALONE : KW_WARPS) * 32)
 knapsack_warp_kernel(const float* __restrict__ scores, int64_t row_stride, int n_rows, int len,
                      const float* __restrict__ budget, KnapOpts o, int max_iters, float tol, float* __restrict__ lam0_out,
                      int* __restrict__ ndbl_out, int64_t* __restrict__ out) {
-  const int b = blockIdx.x * KW_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (b >= n_rows) return;
+  __shared__ float s_lam0[KW_ALONE];
+  __shared__ int s_ndbl[KW_ALONE];
+  const int b = ALONE ? threadIdx.x >> 5 : blockIdx.x * KW_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (b >= n_rows) return;                                  // (ALONE: exactly n_rows warps)
   const float* row = scores + (int64_t)b * row_stride;
   float s[PER];
   float mx = -INFINITY;
@@ -365,8 +372,26 @@ knapsack_warp_kernel(const float* __restrict__ scores, int64_t row_stride, int n
     if (!above(sweep(lam), len, bud)) break;
     lam = __fmul_rn(lam, 2.0f);
   }
-  if (lane == 0) { lam0_out[b] = lam0; ndbl_out[b] = k; }
-  float lam_lo = 0.f, lam_hi = ldexpf(lam0, k), lam_final = 0.f;
+  int rounds = 40;
+  if (ALONE) {
+    if (lane == 0) { s_lam0[b] = lam0; s_ndbl[b] = k; }
+    __syncthreads();
+    if (k >= 2 && ldexpf(lam0, k - 1) >= 1e12f) {           // (only then can the others have ended this row's doublings)
+      rounds = 0;
+      for (; rounds < 40; ++rounds) {
+        bool need = false, big = true;
+        for (int r = 0; r < n_rows; ++r) {
+          need = need || s_ndbl[r] > rounds;
+          big = big && ldexpf(s_lam0[r], min(rounds + 1, s_ndbl[r])) >= 1e12f;
+        }
+        if (!need) break;
+        if (big) { ++rounds; break; }
+      }
+    }
+  } else if (lane == 0) {
+    lam0_out[b] = lam0; ndbl_out[b] = k;
+  }
+  float lam_lo = 0.f, lam_hi = ldexpf(lam0, min(rounds, k)), lam_final = 0.f;
   if (above(sweep(0.f), len, bud)) {
     float lam_mid = 0.f;
 #pragma unroll 1
@@ -614,11 +639,11 @@ static int fill_options(KnapOpts& o, const float* option_bits, const float* opti
 
 static int launch_warp_rows(const float* scores, int64_t row_stride, int n_rows, int len, const float* budget,
                             const KnapOpts& o, int max_iters, float tol, float* lam0, int* ndbl, int64_t* out, cudaStream_t st) {
-  const int grid = (n_rows + KW_WARPS - 1) / KW_WARPS;
-  if (len <= 128)
-    knapsack_warp_kernel<4><<<grid, KW_WARPS * 32, 0, st>>>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, lam0, ndbl, out);
-  else
-    knapsack_warp_kernel<8><<<grid, KW_WARPS * 32, 0, st>>>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, lam0, ndbl, out);
+  const bool alone = n_rows <= KW_ALONE;
+  const int grid = alone ? 1 : (n_rows + KW_WARPS - 1) / KW_WARPS, threads = (alone ? n_rows : KW_WARPS) * 32;
+  const auto kernel = len <= 128 ? (alone ? knapsack_warp_kernel<4, true> : knapsack_warp_kernel<4, false>)
+                                 : (alone ? knapsack_warp_kernel<8, true> : knapsack_warp_kernel<8, false>);
+  kernel<<<grid, threads, 0, st>>>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, lam0, ndbl, out);
   return launch_status();
 }
 
@@ -719,7 +744,7 @@ static int knapsack_batched(const float* scores, int64_t row_stride, int n_rows,
            : cluster == 4 ? launch_bucket_rows<4>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, chunk, lam0, ndbl, out, st)
            : cluster == 2 ? launch_bucket_rows<2>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, chunk, lam0, ndbl, out, st)
                           : launch_bucket_rows<1>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, chunk, lam0, ndbl, out, st);
-    if (rc != RDKV_OK) return rc;
+    if (rc != RDKV_OK || (len <= 256 && n_rows <= KW_ALONE)) return rc;
     knapsack_cut_kernel<<<1, KNAP_THREADS, 0, st>>>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, lam0, ndbl, out);
     return launch_status();
   }

@@ -70,6 +70,23 @@ def test_allocator_lengths(length, kind):
         assert np.array_equal(to_np(got), want)
 
 
+@pytest.mark.parametrize("rows", [1, 2, 16, 17])
+@pytest.mark.parametrize("length", [1, 40, 128, 129, 256])
+def test_short_rows_end_their_doublings_together(rows, length):
+    """One CTA takes up to 16 short rows and replays the batch-wide exit of the doubling loop: rows that can
+    never meet their budget alone, and next to rows that can."""
+    from oracle.ref_knapsack import knapsack_batched
+    from rdkv_b200 import synth
+    from rdkv_b200.knapsack_solver import knapsack_bit_allocation_batched
+    s = synth.make_scores(rows, length, seed=rows + length)
+    s[::2] *= 1e6
+    opts = torch.tensor([2., 4., 8., 16.])
+    for budget in (torch.ones(rows), 1.0 + 3.0 * (torch.arange(rows) % 3).float()):
+        got = knapsack_bit_allocation_batched(s.cuda(), budget.cuda(), epsilon=synth.ALLOC_EPSILON, max_iters=20, bit_options=opts)
+        want = knapsack_batched(s.numpy(), budget.numpy(), synth.ALLOC_EPSILON, max_iters=20, bit_options=(2, 4, 8, 16))
+        assert np.array_equal(to_np(got), want)
+
+
 @pytest.mark.parametrize("length", [1, 2, 3, 1000, 32768, 40001])
 def test_budgets_and_logical_bits(length):
     from oracle.ref_blockwise import logical_layer_bits
