@@ -139,7 +139,14 @@ class DecodeTable:
     ROW_COST = 17.6
     FIXED_WHOLE = 13000.0
     FIXED_CHUNK = 11000.0
-    MERGE_PER_CHUNK = 1500.0             # per chunk of a unit: its record read back by the unit's last CTA, contention on the counter
+    # per chunk of a unit: its record read back by the unit's last CTA, and what a CTA more costs the others on
+    # its SM.  The first figure is for launches of several rounds.  Where one round holds all chunks the SMs
+    # are not full, and more and shorter chunks were faster until they filled the slots (us with the
+    # chunks that the first figure gives -> with the second's; 8 heads, inputs not in L2): 1061 rows 22 in 3
+    # -> 18 in 9, 2565 rows 27 in 6 -> 22 in 14, 8581 rows 36 in 8 -> 31 in 14; four sequences of 2565 rows
+    # 29 in 6 -> 27 in 11; 64 units and more: the same plans.
+    MERGE_PER_CHUNK = 1500.0
+    MERGE_ONE_ROUND = 300.0
 
     def refresh(self) -> None:
         """Rebuild the table's snapshot of the per-head quantities (one small launch on the current
@@ -185,11 +192,12 @@ class DecodeTable:
             cr = self.chunk_rows if (self.chunk_rows and self.chunk_rows * k >= rows) else self._chunk_rows_for(k, rows)
             return k, cr, (units if k == 1 else 0)
         slots = self._sms * self.CTAS_PER_SM
-        k_max = max(1, min(16, rows // 128))
+        k_max = max(1, min(16, -(-rows // 128)))
         whole = rows * self.ROW_COST + self.FIXED_WHOLE
 
         def chunk_cost(k):                                  # (the unit's last CTA also reads all k records)
-            return self._chunk_rows_for(k, rows) * self.ROW_COST + self.FIXED_CHUNK + k * self.MERGE_PER_CHUNK
+            merge = self.MERGE_ONE_ROUND if units * k <= slots else self.MERGE_PER_CHUNK
+            return self._chunk_rows_for(k, rows) * self.ROW_COST + self.FIXED_CHUNK + k * merge
 
         best = (-(-units // slots) * whole, 1, units)                       # all whole
         full, left = divmod(units, slots)

@@ -77,6 +77,24 @@ def test_tail_tiles(counts, tails, dtype):
             assert_attn_close(to_np(out[i]), want, f"view {i}, chunks {n_chunks}")
 
 
+@pytest.mark.parametrize("rows", [128, 129, 257, 1061, 2600])
+@pytest.mark.parametrize("counts", [(16, 24, 24), (23, 31, 35)])
+def test_few_units_in_many_chunks(rows, counts):
+    """A launch of few units is cut into up to 16 chunks each, the last of them short or empty: against
+    whole units."""
+    from rdkv_b200 import synth
+    from rdkv_b200.decode import DecodeTable, packed_decode_attention
+    g, H = 4, 2
+    pl, nv = _layer(counts, rows + 20, [rows, max(1, rows // 3)], 7, g)
+    q = synth.make_q(H * g, seed=8, batch=1).cuda()
+    table = DecodeTable([pl], [nv], H * g)
+    k, chunk, n_whole = table.plan(1)
+    assert k * chunk >= rows and k <= 16 and (n_whole == 0) == (k > 1)
+    whole = packed_decode_attention(q, DecodeTable([pl], [nv], H * g, n_chunks=1))
+    assert_attn_close(to_np(packed_decode_attention(q, table)), to_np(whole), f"{k} chunks of {chunk}")
+    table.check_status()
+
+
 @pytest.mark.parametrize("rows", [1, 127, 128, 255, 256, 700, 2048])
 @pytest.mark.parametrize("heads,g", [(1, 4), (2, 8), (8, 4), (3, 16)])
 def test_weighted_sum_in_clusters(rows, heads, g):
