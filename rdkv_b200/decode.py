@@ -120,9 +120,9 @@ class DecodeTable:
         if not self.live_counts:
             recs = self.unit_recs.view(torch.int32).view(n_units, self._unit_rec_bytes // 4)
             # (bit 1: the V rows come through tensor maps; bit 2: K rows of one span per segment on whole words)
-            flags = recs[:, 4]
-            self._all_fast, simple = torch.stack([((flags & 3) == 3).all(), ((flags & 4) != 0).all()]).tolist()
-            self._wide = not simple
+            flags = recs[:, 4].cpu().numpy()
+            self._all_fast = bool(((flags & 3) == 3).all())
+            self._wide = not ((flags & 4) != 0).all()
         self.k_rows_arg = self.k_row_bytes_max | (RDKV_K_ANY_ROWS if self._wide else 0)
 
     CTAS_PER_SM = 3                      # resident CTAs of the fused kernel per SM
