@@ -597,14 +597,14 @@ def run_pack(args, rank, world, device):
     with sampler:
         ms = timed_steps(step, args.steps, lambda: None)
     sec = ms / 1e3 / args.steps
-    # the launches alone (device time of the two partition and the two packing kernels), for the roofline
+    # the launches alone (device time of the partition and the two packing kernels), for the roofline
     spans = []
     torch.cuda.profiler.start()
     for i in range(args.steps):
         state["batch"] = pack_kv_layers(Ks, Vs, v_bits, k_bits, 4, build_mask=False, k_passes=args.k_passes, launch_events=spans)
     torch.cuda.synchronize()
     torch.cuda.profiler.stop()
-    # per call two spans: the two partition launches, the packing launches (V pass, one-pass K)
+    # per call two spans: the partition launch, the packing launches (V pass, one-pass K)
     kern_ms = sum(a.elapsed_time(b) for a, b in spans) / args.steps
     out_bytes = 0
     for pl, nv in state["batch"]:
@@ -626,7 +626,7 @@ def run_pack(args, rank, world, device):
             "roofline": {"bound": "hbm", "achieved": moved / (kern_ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": moved / (kern_ms / 1e3) / 1e9 / peak,
                          "traffic": PACK_NCU_TRAFFIC_BYTES, "peak_kind": kind,
-                         "kernel": "2 x partition_kernel + pack_v128_batched_kernel + pack_k_onepass_batched_kernel",
+                         "kernel": "partition_pair_kernel + pack_v128_batched_kernel + pack_k_onepass_batched_kernel",
                          "kernel_ms": kern_ms, "algorithmic_bytes_per_step": moved},
             "gpu_launches": 4 * 2 * args.steps, "clocks": sampler.summary()}
     if not args.no_cpu_baseline:
@@ -737,7 +737,7 @@ def run_alloc(args, rank, world, device):
                                             "l2": "latency/ALU-bound; inputs 34 MB"},
             "roofline": {"bound": "hbm", "achieved": bytes_ / sec / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": bytes_ / sec / 1e9 / peak, "traffic": None, "peak_kind": kind,
-                         "kernel": "knapsack_seed_kernel + knapsack_solve_kernel",
+                         "kernel": "knapsack_bucket_kernel + knapsack_warp_kernel",
                          "note": "scores read once (4 B) + int64 decisions written (8 B); the kernel is ALU/latency-bound"},
             "gpu_launches": 4 * args.steps, "clocks": sampler.summary()}
     if not args.no_cpu_baseline:

@@ -148,8 +148,8 @@ int rdkv_v_weighted_sum(const rdkv_layer_view* view, const float* w, int64_t w_r
  * rdkv_decode_weighted_sum — what v_dequant_weighted_sum_dispatch_into computes
  * (obkv_accel/triton_v_kernel.py:1729-1760): out[h][:] = sum_t weights[h][t] * V^[t]
  * with weight columns = stripe rows; out fp32 [H_q][128] contiguous; K is not read;
- * unit_rows >= the longest head's live rows (one CTA per KV head, fixed summation
- * order). */
+ * unit_rows >= the longest head's live rows (a cluster of CTAs per KV head, fixed
+ * summation order). */
 int rdkv_decode_scores(const rdkv_layer_view* views, int n_views, const void* q, int q_dtype, int H_q,
                        int H_kv, int chunk_rows, int n_chunks, int k_row_bytes_max, int t_eff,
                        float* scores, int64_t scores_row_stride, int32_t* status, void* stream);

@@ -46,9 +46,6 @@ __device__ __forceinline__ float quant_code_fast_f(float x, float rinv, const QP
   if (fabsf(__fsub_rn(yc, c)) > 0.5f - 1.3e-4f) return (float)quant_code(x, p);
   return c;
 }
-__device__ __forceinline__ unsigned quant_code_fast(float x, float rinv, const QParam& p) {
-  return (unsigned)quant_code_fast_f(x, rinv, p);
-}
 
 // Codes of N values at once (as exact small floats), with ONE branch to the exact path for all of them: a
 // branch per value costs more instructions than its code does (pack_k_quant_body, 4 layers x 8 heads x 8192
