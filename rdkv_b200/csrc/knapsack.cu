@@ -87,7 +87,9 @@ __device__ const float* stage_row(const float* grow, int len, float* smem_row, b
 // 256 rows x 32768: 94 us (every element in every sweep, two kernels: 371).
 // (Tried and slower, times of a whole call with its channel rows while it took 205 us: thresholds worked out by
 // one warp and runs of buckets between them tested, 230; a first test per octave, 231; three multipliers a
-// sweep, 480.)
+// sweep, 480.  Later, kernel alone: buckets whose choice is the same at both ends of the multiplier's interval
+// left out of later sweeps, 96 instead of 91; the scores kept in registers for the sort, 88 here but 43
+// instead of 40 for 8 rows.)
 // A row is spread over a cluster of CTAs (each sorts its own part; partial sums meet in every CTA's shared
 // memory), so that a few rows still fill the chip and a row of 262144 fits.
 // What a sum of chosen bits means for the search: 0 = within `tol` of the budget, 1 = above it, -1 = not above.
