@@ -126,8 +126,11 @@ constexpr int KB_BUCKETS = 1024;
 constexpr int KB_SHIFT = 18;                                // float bits below the bucket number: 5 mantissa bits stay
 constexpr int KB_MAX_CLUSTER = 8;
 constexpr int KB_MAX_CHUNK = 32768;                         // elements per CTA
+constexpr int KB_SMALL_CHUNK = 16384;                       // up to here with 512 threads, above with 1024
 constexpr int KB_PIECE = 64;                                // elements a warp takes at a time
 constexpr int KB_BATCH = 4;                                 // loads in flight per thread
+// dynamic shared memory: the part's scores in bucket order and the list of pieces to look at
+__host__ __device__ constexpr size_t kb_smem_bytes(int chunk) { return (size_t)chunk * 4 + ((size_t)KB_BUCKETS + chunk / KB_PIECE) * 4; }
 
 template <int KB_THREADS>
 struct KnapShared {
@@ -655,9 +658,12 @@ template <int S, int THREADS>
 static int launch_bucket_rows_of(const float* scores, int64_t row_stride, int n_rows, int len, const float* budget,
                               const KnapOpts& o, int max_iters, float tol, int chunk, float* lam0, int* ndbl, int64_t* out,
                               cudaStream_t st) {
-  const size_t smem = (size_t)chunk * 4 + ((size_t)KB_BUCKETS + chunk / KB_PIECE) * 4;
+  const size_t smem = kb_smem_bytes(chunk);
   if ((int64_t)n_rows * S > 0x7fffffffLL) return RDKV_ERR_TOO_LARGE;
-  cudaError_t e = cudaFuncSetAttribute(knapsack_bucket_kernel<S, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // (the limit belongs to the function, not to this launch: every call sets the same one, that of the longest part
+  //  the instance takes, so that a call from another thread cannot lower it between here and the launch)
+  constexpr int limit = (int)kb_smem_bytes(THREADS == 1024 ? KB_MAX_CHUNK : KB_SMALL_CHUNK);
+  cudaError_t e = cudaFuncSetAttribute(knapsack_bucket_kernel<S, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
   if (e == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_rows * S);
@@ -679,7 +685,7 @@ template <int S>
 static int launch_bucket_rows(const float* scores, int64_t row_stride, int n_rows, int len, const float* budget,
                               const KnapOpts& o, int max_iters, float tol, int chunk, float* lam0, int* ndbl, int64_t* out,
                               cudaStream_t st) {
-  return (chunk > 16384 ? launch_bucket_rows_of<S, 1024> : launch_bucket_rows_of<S, 512>)(
+  return (chunk > KB_SMALL_CHUNK ? launch_bucket_rows_of<S, 1024> : launch_bucket_rows_of<S, 512>)(
       scores, row_stride, n_rows, len, budget, o, max_iters, tol, chunk, lam0, ndbl, out, st);
 }
 
@@ -717,13 +723,6 @@ static int knapsack_batched(const float* scores, int64_t row_stride, int n_rows,
   const int orc = fill_options(o, option_bits, option_eps, n_options, len);
   if (orc != RDKV_OK) return orc;
   o.budget = budget_all;
-  const size_t row_bytes = (size_t)len * sizeof(float);
-  const int use_smem = row_bytes <= (size_t)KNAP_SMEM_ROW_BYTES ? 1 : 0;
-  const size_t smem = use_smem ? row_bytes : 0;
-  if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(knapsack_seed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KNAP_SMEM_ROW_BYTES);
-    cudaFuncSetAttribute(knapsack_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KNAP_SMEM_ROW_BYTES);
-  }
   float* lam0 = reinterpret_cast<float*>(scratch);
   int* ndbl = reinterpret_cast<int*>(lam0 + 2 * (size_t)n_rows);
   cudaStream_t st = (cudaStream_t)stream;
@@ -751,6 +750,13 @@ static int knapsack_batched(const float* scores, int64_t row_stride, int n_rows,
     if (rc != RDKV_OK || (len <= 256 && n_rows <= KW_ALONE)) return rc;
     knapsack_cut_kernel<<<1, KNAP_THREADS, 0, st>>>(scores, row_stride, n_rows, len, budget, o, max_iters, tol, lam0, ndbl, out);
     return launch_status();
+  }
+  const size_t row_bytes = (size_t)len * sizeof(float);
+  const int use_smem = row_bytes <= (size_t)KNAP_SMEM_ROW_BYTES ? 1 : 0;
+  const size_t smem = use_smem ? row_bytes : 0;
+  if (smem > 48 * 1024) {
+    cudaFuncSetAttribute(knapsack_seed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KNAP_SMEM_ROW_BYTES);
+    cudaFuncSetAttribute(knapsack_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KNAP_SMEM_ROW_BYTES);
   }
   knapsack_seed_kernel<<<n_rows, KNAP_THREADS, smem, st>>>(scores, row_stride, len, budget, o, use_smem, lam0, ndbl);
   int rc = launch_status();
