@@ -145,9 +145,11 @@ extern "C" int rdkv_block_scores(const void* queries, int q_dtype, int64_t q_hea
   if (causal && Q != T) return RDKV_ERR_BAD_SHAPE;
   if (H_kv == 0) return RDKV_OK;
   const int span = T > D ? T : D;
-  const size_t smem =
-      sizeof(float) * ((size_t)T * (D + 1) + (size_t)BS_WARPS * D + (size_t)BS_WARPS * span + 2 * (size_t)span);
-  cudaError_t e = cudaFuncSetAttribute(block_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto smem_bytes = [](int T, int D, int span) {
+    return sizeof(float) * ((size_t)T * (D + 1) + (size_t)BS_WARPS * D + (size_t)BS_WARPS * span + 2 * (size_t)span);
+  };
+  const size_t smem = smem_bytes(T, D, span);
+  cudaError_t e = allow_dynamic_smem(block_score_kernel, smem_bytes(BS_MAX_T, 128, BS_MAX_T));
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(H_kv * BS_CLUSTER);

@@ -325,7 +325,7 @@ extern "C" int rdkv_v_weighted_sum(const rdkv_layer_view* view, const float* w, 
   const int g = H_q / H_kv;
   const size_t smem = sizeof(float) * (VSUM_THREADS / 32) * GP * D;
   // (per device, not per process: set on every call, as the fused kernel's launcher does)
-  cudaError_t e = cudaFuncSetAttribute(v_weighted_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dynamic_smem(v_weighted_sum_kernel, smem);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
   v_weighted_sum_kernel<<<H_kv, VSUM_THREADS, smem, (cudaStream_t)stream>>>(*view, w, w_row_stride, g, out,
                                                                            out_row_stride);

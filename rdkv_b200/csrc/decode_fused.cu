@@ -63,6 +63,7 @@ constexpr int DPAD_MAX = RDKV_DPAD_MAX;  // padded channel slots of a view (n_ch
 // (those three only in launches without a prepared table)
 constexpr int FOLD_Q_BYTES = GH * 128 * 4;
 constexpr int FOLD_META_BYTES = 3 * DPAD_MAX * 2;
+constexpr int K_ROW_BYTES_MOST = 224;  // K bytes of a row: 128 channels in each segment
 constexpr float TWO24 = 16777216.f;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
@@ -110,7 +111,7 @@ static_assert(phase_tile_rows(0) * phase_pitch(0) <= V_STAGE && phase_tile_rows(
               "a tile's V rows fit the V area at their padded pitch");
 
 __host__ __device__ inline int align16i(int x) { return (x + 15) & ~15; }
-__host__ __device__ inline int align128i(int x) { return (x + 127) & ~127; }
+__host__ __device__ constexpr int align128i(int x) { return (x + 127) & ~127; }
 
 struct StageLayout {                   // byte offsets inside one stage
   int v, k2, k4, k8, sc, zp, total;
@@ -128,7 +129,7 @@ __host__ __device__ inline StageLayout stage_layout(int sub2, int sub4, int n8) 
   return L;
 }
 
-__host__ __device__ inline int stage_capacity(int k_row_bytes_max) {
+__host__ __device__ constexpr int stage_capacity(int k_row_bytes_max) {
   return V_STAGE + 32 + TILE_MAX * k_row_bytes_max + 3 * 64 + 2 * (TILE_MAX * 2 + 32);
 }
 
@@ -1930,7 +1931,10 @@ static int launch_fused(const rdkv_layer_view* views, int n_views, const void* q
   TailArgs ta;
   memset(&ta, 0, sizeof(ta));
   if (tail != nullptr) ta = *tail;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t most = (size_t)FSTAGES * align128i(stage_capacity(K_ROW_BYTES_MOST)) + KB_MAX * 256 + FOLD_Q_BYTES +
+                          FOLD_META_BYTES + (MODE == MODE_ATTN_TAIL ? TAIL_EXTRA_BYTES : 0);
+  static_assert(most <= 215 * 1024, "with the static shared memory within an SM's 227 KB");
+  cudaError_t e = allow_dynamic_smem(kernel, most);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)items);
@@ -1958,7 +1962,7 @@ static int check_fused_args(const rdkv_layer_view* views, int n_views, const voi
   if (q_dtype < RDKV_F16 || q_dtype > RDKV_F32) return RDKV_ERR_BAD_ARG;
   if (H_q <= 0 || H_kv <= 0 || H_q % H_kv != 0) return RDKV_ERR_BAD_SHAPE;
   k_row_bytes_max &= ~RDKV_K_ANY_ROWS;
-  if (k_row_bytes_max <= 0 || k_row_bytes_max > 224) return RDKV_ERR_BAD_SHAPE;
+  if (k_row_bytes_max <= 0 || k_row_bytes_max > K_ROW_BYTES_MOST) return RDKV_ERR_BAD_SHAPE;
   return RDKV_OK;
 }
 
@@ -2190,7 +2194,10 @@ extern "C" int rdkv_decode_attn_persistent(const rdkv_layer_view* views, int n_v
   const size_t epilogue = (size_t)FW * GH * D * sizeof(float);
   if ((size_t)stage_bytes < epilogue) return RDKV_ERR_BAD_SHAPE;     // the merge works inside one ring slot
   if (smem > 227 * 1024) return RDKV_ERR_TOO_LARGE;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t most = (size_t)FSTAGES * align128i(stage_capacity(K_ROW_BYTES_MOST)) + KB_MAX * 256 +
+                          2 * ((size_t)GH * D * 4 + (size_t)KB_MAX * KSLOT_RECS * sizeof(KSlotRec));
+  static_assert(most <= 215 * 1024, "with the static shared memory within an SM's 227 KB");
+  cudaError_t e = allow_dynamic_smem(kernel, most);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||

@@ -660,10 +660,8 @@ static int launch_bucket_rows_of(const float* scores, int64_t row_stride, int n_
                               cudaStream_t st) {
   const size_t smem = kb_smem_bytes(chunk);
   if ((int64_t)n_rows * S > 0x7fffffffLL) return RDKV_ERR_TOO_LARGE;
-  // (the limit belongs to the function, not to this launch: every call sets the same one, that of the longest part
-  //  the instance takes, so that a call from another thread cannot lower it between here and the launch)
-  constexpr int limit = (int)kb_smem_bytes(THREADS == 1024 ? KB_MAX_CHUNK : KB_SMALL_CHUNK);
-  cudaError_t e = cudaFuncSetAttribute(knapsack_bucket_kernel<S, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+  // (the size of the longest part the instance takes)
+  cudaError_t e = allow_dynamic_smem(knapsack_bucket_kernel<S, THREADS>, kb_smem_bytes(THREADS == 1024 ? KB_MAX_CHUNK : KB_SMALL_CHUNK));
   if (e == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_rows * S);

@@ -681,8 +681,9 @@ static int obs_scores(const void* q_obs, const void* k, int dtype, int64_t q_hea
   const size_t smem = 1024 + (size_t)(2 + MB) * OBS_BLOCK;   // (the base is rounded up to 1024 bytes in the kernel)
   cudaStream_t st = (cudaStream_t)stream;
   auto launch = [&](auto kern_stats, auto kern_token) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern_stats, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern_token, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t most = 1024 + (size_t)(2 + OBS_MAX_ROWS / OBS_ROWS) * OBS_BLOCK;
+    cudaError_t e = allow_dynamic_smem(kern_stats, most);
+    if (e == cudaSuccess) e = allow_dynamic_smem(kern_token, most);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
     kern_stats<<<dim3(A.P, BH), OBS_THREADS, smem, st>>>(A, tm_q, tm_k);
     int rc = launch_status();

@@ -1197,7 +1197,7 @@ extern "C" int rdkv_pack_k(const uint16_t* K, int64_t k_head_stride, int64_t k_r
   rc = launch_status();
   if (rc != RDKV_OK) return rc;
   const size_t smem = pack_k_quant_smem(d_pad, A.stage_rows != 0);
-  if (cudaFuncSetAttribute(pack_k_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (allow_dynamic_smem(pack_k_quant_kernel, pack_k_quant_smem(PACKK_MAX_DPAD, true)) != cudaSuccess)
     return launch_status();
   pack_k_quant_kernel<<<dim3(pack_k_quant_ctas(t_k, H), H), PACKK_WARPS * 32, smem, st>>>(A);
   return launch_status();
@@ -1228,8 +1228,7 @@ static int pack_kv_jobs(const Jobs& jobs, int n_jobs, int H, int D, int max_slot
   const bool one_fits = D == 128 && one_smem <= (size_t)KOP_MAX_SMEM;
   if (k_passes == 1 && !one_fits) return RDKV_ERR_TOO_LARGE;
   if (one_fits && (k_passes == 1 || (k_passes == 0 && one_smem <= (size_t)KOP_AUTO_SMEM))) {
-    cudaError_t e = cudaFuncSetAttribute(pack_k_onepass_batched_kernel<Jobs>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)one_smem);
+    cudaError_t e = allow_dynamic_smem(pack_k_onepass_batched_kernel<Jobs>, KOP_MAX_SMEM);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return RDKV_ERR_LAUNCH; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(KOP_CL, H, n_jobs);
@@ -1253,7 +1252,7 @@ static int pack_kv_jobs(const Jobs& jobs, int n_jobs, int H, int D, int max_slot
   rc = launch_status();
   if (rc != RDKV_OK) return rc;
   const size_t smem = pack_k_quant_smem(max_d_pad, D == 128);
-  if (cudaFuncSetAttribute(pack_k_quant_batched_kernel<Jobs>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (allow_dynamic_smem(pack_k_quant_batched_kernel<Jobs>, pack_k_quant_smem(PACKK_MAX_DPAD, true)) != cudaSuccess)
     return launch_status();
   pack_k_quant_batched_kernel<Jobs><<<dim3(pack_k_quant_ctas(max_t_k, (int64_t)H * n_jobs), H, n_jobs), PACKK_WARPS * 32, smem, st>>>(jobs);
   return launch_status();

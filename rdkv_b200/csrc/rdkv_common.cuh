@@ -17,6 +17,14 @@ constexpr int MAX_GROUP = 16;                        // query heads per KV head
 // Per-thread record of the last failed launch, read back by rdkv_last_cuda_error().
 extern thread_local int g_last_cuda_error;
 
+// Raises a kernel's limit of dynamic shared memory.  The limit belongs to the function on this device, not to a
+// launch: `most` is the same in every call for a kernel (the largest size its launcher can ask for), so that a
+// call from another thread never lowers it between this one and its launch.
+template <class Kernel>
+inline cudaError_t allow_dynamic_smem(Kernel kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 inline int launch_status() {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
