@@ -173,9 +173,9 @@ def _fill_view(v: LayerView, pl: PackedKVLayer, V16: Optional[Tensor], rows: int
     return keep
 
 
-def _unpack_layers(layers, V16s, D: int) -> List[Tuple[Tensor, Tensor]]:
+def _unpack_layers(layers, V16s, D: int, first: int = 0) -> List[Tuple[Tensor, Tensor]]:
     """(K, V) fp16 stripes of every layer, the fp16-V rows included: ``unpack_k_mixed`` and ``_v_stripe``
-    of all of them in one call."""
+    of all of them in one call.  ``first``: the number of the first of them in its cache."""
     jobs = (UnpackJob * max(1, len(layers)))()
     out, keep, n = [], [], 0
     devices = set()
@@ -188,7 +188,7 @@ def _unpack_layers(layers, V16s, D: int) -> List[Tuple[Tensor, Tensor]]:
         rows_k = int(pl.T_eff_k) if pl.T_eff_k > 0 else int(pl.T_eff)
         n16 = int(pl.n_v16) if _is_perhead_layout(pl) else (int(V16.shape[2]) if V16 is not None and V16.numel() > 0 else 0)
         rows = int(pl.T_eff) + n16
-        assert rows_k == rows, (f"layer {i}: K T-dim {rows_k} != V T-dim {rows} "
+        assert rows_k == rows, (f"layer {first + i}: K T-dim {rows_k} != V T-dim {rows} "
                                 f"(T_v={pl.T_eff}, n_v16={pl.n_v16}, T_eff_k={pl.T_eff_k})")
         si, stride, cnt, n_ch = _k_channel_maps(pl)
         no_k = si is None or sum(n_ch) == 0
@@ -224,11 +224,22 @@ def unpack_trizone_to_past_kv(dual_cache: TriZoneCache, *, head_dim: int, device
     """Reverse a ``TriZoneCache`` into HF legacy ``past_key_values``: a tuple of ``(K_i, V_i)``, each
     ``[1, H_kv, T_eff_k_i, head_dim]``; with ``return_masks`` also the per-layer ``[1, H_q, 1,
     T_eff_k_i + max_new_tokens]`` additive masks of the per-head layout (``None`` for shared-layout
-    layers).  Same contract as trizone_decompress.py:185-333."""
+    layers).  Same contract as trizone_decompress.py:185-333.
+
+    Stripes that stay as they are unpacked (no other ``device`` or ``dtype``) are the result and come from
+    one launch per 16 layers.  Stripes that are moved or converted are unpacked and let go one layer at a
+    time: a cache that does not fit the GPU in fp16 can be unpacked to the host."""
     past_kv: List[Tuple[Tensor, Tensor]] = []
     masks_list: List[Optional[Tensor]] = []
-    V16s = [dual_cache.new_v_only[i] if i < len(dual_cache.new_v_only) else None for i in range(len(dual_cache.packed))]
-    for i, (pl, (K_full, V_full)) in enumerate(zip(dual_cache.packed, _unpack_layers(dual_cache.packed, V16s, head_dim))):
+    layers = list(dual_cache.packed)
+    V16s = [dual_cache.new_v_only[i] if i < len(dual_cache.new_v_only) else None for i in range(len(layers))]
+    target = None if device is None else torch.device(device)
+    stay = dtype == torch.float16 and (target is None or all(
+        pl.K_ch_scale is not None and target.type == pl.K_ch_scale.device.type
+        and target.index in (None, pl.K_ch_scale.device.index) for pl in layers))
+    dense = _unpack_layers(layers, V16s, head_dim) if stay else None
+    for i, pl in enumerate(layers):
+        K_full, V_full = dense[i] if stay else _unpack_layers([pl], V16s[i:i + 1], head_dim, i)[0]
         per_head = _is_perhead_layout(pl)
         if device is not None:
             K_full, V_full = K_full.to(device), V_full.to(device)
