@@ -584,16 +584,16 @@ int rdkv_knapsack_rows(const float* scores, int64_t row_stride, int n_rows, int 
 
 /* ── batched bit allocator without caller-provided scratch ────────────────────
  * No counterpart in the reference.  Same computation and arguments as
- * rdkv_knapsack_batched, minus `scratch`: the three words per row the two kernels
+ * rdkv_knapsack_batched, minus `scratch`: the three words per row that its kernels
  * hand over to each other live in a fixed array inside the library's device image
  * (48 KiB on every GPU that loads the library, held until the process exits).  It is
  * meant for callers that may not allocate device memory where they call from — an
  * engine that froze its memory plan after warm-up, or a plugin that is given input
- * and output buffers and nothing else.  After one warm-up call per device the call
- * performs no allocation of any kind (the first call on a device makes the runtime
- * load the library's module there, which reserves device memory, and opts the
- * kernels into large shared memory if the row is longer than 48 KiB: warm up before
- * the memory plan is frozen, with a row as long as the longest that will follow).
+ * and output buffers and nothing else.  After one warm-up call per device, of any
+ * shape, the call performs no allocation of any kind, whatever shapes follow (the
+ * first call on a device makes the runtime load the library's module there and every
+ * kernel that any shape may use, which reserves device memory: warm up before the
+ * memory plan is frozen).
  *   - n_rows above rdkv_knapsack_static_max_rows() (4096) is refused with
  *     RDKV_ERR_TOO_LARGE; split the batch or use rdkv_knapsack_batched.
  *   - The first call on each device looks up the array's device address

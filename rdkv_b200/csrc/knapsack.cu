@@ -788,9 +788,9 @@ extern "C" int rdkv_knapsack_batched_uniform(const float* scores, int64_t row_st
 // For them the scratch lives in this library's own device image: a file-scope
 // array that every GPU loading the library carries until the process exits.
 // (One warm-up call per device, made before the memory plan is frozen and before any
-// stream capture, looks the array's address up and lets the runtime load the module;
-// rows longer than 48 KiB also opt the kernels into large shared memory on that call,
-// so the warm-up should use a row as long as the longest that will follow.)
+// stream capture, looks the array's address up and lets the runtime load the module
+// and every kernel that a call of any shape may choose: with lazy loading a kernel's code
+// would otherwise be loaded by the first launch of it.)
 constexpr int KNAP_STATIC_MAX_ROWS = 4096;                 // 3 words per row -> 48 KiB per GPU
 static __device__ __align__(256) unsigned int g_knap_static_scratch[3 * KNAP_STATIC_MAX_ROWS];
 
@@ -800,6 +800,23 @@ constexpr int KNAP_MAX_DEVICES = 64;
 std::mutex g_knap_static_mutex;
 void* g_knap_static_addr[KNAP_MAX_DEVICES] = {nullptr};   // device address of the array, per device
 }  // namespace
+
+template <typename... Kernels>
+static cudaError_t load_kernels(Kernels... kernels) {
+  cudaError_t e = cudaSuccess;
+  cudaFuncAttributes attr;
+  ((e = e == cudaSuccess ? cudaFuncGetAttributes(&attr, kernels) : e), ...);   // (loads the code, lazy or not)
+  return e;
+}
+
+// Every kernel that knapsack_batched chooses from.
+static cudaError_t load_batched_kernels() {
+  return load_kernels(knapsack_bucket_kernel<1, 512>, knapsack_bucket_kernel<2, 512>, knapsack_bucket_kernel<4, 512>,
+                      knapsack_bucket_kernel<8, 512>, knapsack_bucket_kernel<1, 1024>, knapsack_bucket_kernel<2, 1024>,
+                      knapsack_bucket_kernel<4, 1024>, knapsack_bucket_kernel<8, 1024>, knapsack_warp_kernel<4, false>,
+                      knapsack_warp_kernel<4, true>, knapsack_warp_kernel<8, false>, knapsack_warp_kernel<8, true>,
+                      knapsack_cut_kernel, knapsack_seed_kernel, knapsack_solve_kernel);
+}
 
 extern "C" int rdkv_knapsack_static_max_rows(void) { return KNAP_STATIC_MAX_ROWS; }
 
@@ -821,7 +838,8 @@ extern "C" int rdkv_knapsack_batched_static(const float* scores, int64_t row_str
     std::lock_guard<std::mutex> lock(g_knap_static_mutex);
     if (g_knap_static_addr[dev] == nullptr) {
       void* p = nullptr;
-      e = cudaGetSymbolAddress(&p, g_knap_static_scratch);
+      e = load_batched_kernels();
+      if (e == cudaSuccess) e = cudaGetSymbolAddress(&p, g_knap_static_scratch);
       if (e != cudaSuccess || p == nullptr) {
         g_last_cuda_error = (int)e;
         return RDKV_ERR_LAUNCH;

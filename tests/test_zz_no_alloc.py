@@ -11,6 +11,9 @@ The file name sorts last on purpose: a run that stops at the first failure has t
 already been through every other test.
 """
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -58,3 +61,38 @@ def test_static_scratch_variant_matches_regular_entry_point_twice():
     out = torch.empty((4097, 8), dtype=torch.int64, device="cuda")
     bud = torch.full((4097,), 2.0, dtype=torch.float32, device="cuda")
     assert _call(True, big, bud, out, eps) == 3
+
+
+# (rows, length) of every kernel the call chooses from, behind a warm-up of another shape
+SHAPES = [(8, 100), (300, 100), (8, 200), (300, 200), (300, 1000), (100, 5000), (40, 20000), (8, 40000), (300, 20000),
+          (100, 32769), (30, 65537), (8, 131073), (3, 300000)]
+
+CHILD = """
+import sys
+import torch
+from rdkv_b200 import _lib, synth
+from test_zz_no_alloc import SHAPES, _call
+n = max(r * t for r, t in SHAPES)
+scores = torch.rand(n, device="cuda")
+out = torch.empty(n, dtype=torch.int64, device="cuda")
+budget = torch.full((4096,), 2.0, device="cuda")
+def call(rows, length, eps):
+    assert _call(True, scores[:rows * length].view(rows, length), budget[:rows], out, eps) == 0
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+eps = dict(synth.ALLOC_EPSILON)
+free = call(4, 700, eps)
+told = [(r, t, call(r, t, eps)) for r, t in SHAPES]
+eps[8] = -eps[8]                                             # (the kernels for negative distortions)
+told += [(r, t, call(r, t, eps)) for r, t in ((3, 700), (3, 300000))]
+sys.exit(f"{free} bytes free after the warm-up, then {told}" if any(f != free for _, _, f in told) else 0)
+"""
+
+
+def test_one_warm_up_call_loads_every_kernel():
+    """After one call of one shape the device's free memory stays where it is, whatever shapes follow (in a
+    fresh process: what a process has loaded it keeps)."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here]), CUDA_MODULE_LOADING="LAZY")
+    got = subprocess.run([sys.executable, "-c", CHILD], env=env, capture_output=True, text=True, timeout=300)
+    assert got.returncode == 0, got.stdout + got.stderr
