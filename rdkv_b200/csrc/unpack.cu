@@ -113,6 +113,7 @@ constexpr int UP_THREADS = 256;
 constexpr int UP_ROWS = 128;                                 // stripe rows per CTA
 constexpr int UP_JOBS = 16;                                  // layers per launch (their records are launch arguments)
 struct UnpackJobs { rdkv_unpack_job j[UP_JOBS]; };
+constexpr int UP_STATIC_SMEM = 128 * (2 + 4 * 4);            // s_slot, s_where, s_how, s_sc, s_zp of the kernel
 
 // float(code) without a conversion instruction: the code in the mantissa of 2^23, exact.
 __device__ __forceinline__ float code_f(uint32_t bits) { return __uint_as_float(0x4B000000u | bits) - 8388608.f; }
@@ -289,13 +290,15 @@ static size_t unpack_smem(const rdkv_layer_view& v) {
 }
 
 // The 128-channel kernel moves 8-byte words of V codes and 16-byte words of fp16 rows: bases and head
-// strides on those boundaries (what this library packs always is), and K rows that fit its shared memory.
+// strides on those boundaries (what this library packs always is), and K rows that fit its shared memory beside
+// its tables within the 48 KB every launch may have (365 bytes a row; 128 channels take 224 at most, but a layer
+// packed for larger channel targets can be wider).
 static bool unpack_fast(const rdkv_unpack_job& J, int D) {
   const rdkv_layer_view& v = J.view;
   auto al = [](const void* p, int64_t stride_bytes, int a) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)stride_bytes) & (a - 1)) == 0; };
   return D == 128 && al(J.k_out, 2 * J.out_head_stride, 16) && al(J.v_out, 2 * J.out_head_stride, 16) &&
          al(v.v2, v.v2_head_stride, 8) && al(v.v4, v.v4_head_stride, 8) && al(v.v8, v.v8_head_stride, 8) &&
-         al(v.v16, 2 * v.v16_head_stride, 16) && (J.k_out == nullptr || unpack_smem(v) <= 48 * 1024);
+         al(v.v16, 2 * v.v16_head_stride, 16) && (J.k_out == nullptr || unpack_smem(v) + UP_STATIC_SMEM <= 48 * 1024);
 }
 
 extern "C" int rdkv_sizeof_unpack_job(void) { return (int)sizeof(rdkv_unpack_job); }

@@ -168,6 +168,28 @@ def test_unpack_rows(rows, mix):
         assert torch.equal(unpack_k_mixed(pl, 128), k)
 
 
+@pytest.mark.parametrize("n8", [300, 365, 366, 383, 384, 450])
+def test_unpack_wide_rows(n8):
+    """K rows packed for larger channel targets than a head has channels: up to the widest that the
+    128-channel kernel has shared memory for, and wider ones, which the general kernel takes."""
+    from rdkv_b200.decompress import unpack_k_mixed
+    from rdkv_b200.packing import PackedKVLayer, pack_k_mixed
+    H, T = 2, 131
+    K = torch.randn(1, H, T, 128, generator=torch.Generator().manual_seed(n8)).half().cuda()
+    bits = torch.full((128,), 8, device="cuda")
+    none = torch.empty(1, H, 0, 1, dtype=torch.float16, device="cuda")
+
+    def unpacked(target):
+        k2, k4, k8, scale, zp, sort_idx, perm, (_, _, n) = pack_k_mixed(K, bits, n_ch_8_target=target)
+        assert n == 128 and k8.shape[-1] == target
+        layer = PackedKVLayer(k2, k4, k8, scale, zp, sort_idx, (0, 0, target), perm, None, None, None, none, none, sort_idx[:0],
+                              (0, 0, 0), 0, T_eff_k=T, K_ch_sort_idx_per_head=sort_idx.repeat(H, 1),
+                              K_ch_seg_bounds_per_head=torch.tensor([[0, 0, 128]] * H, dtype=torch.int32, device="cuda"))
+        return unpack_k_mixed(layer, 128)
+
+    assert torch.equal(unpacked(n8), unpacked(128))
+
+
 @pytest.mark.parametrize("tokens,window,g", [(33, 32, 4), (128, 8, 4), (129, 16, 8), (1000, 32, 8), (5000, 5, 3)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_normalised_window_scores(tokens, window, g, causal):
