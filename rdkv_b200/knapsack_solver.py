@@ -157,6 +157,10 @@ def k_budgets_from_v_bits(token_budget: int, head_dim: int, k_budget_ratio: floa
     """:func:`k_average_bits_per_head` of the tokens kept in every row of ``v_bits`` [H,T] (the V
     allocation's result on the GPU): the same fp32 values, counted and divided in one launch."""
     require_cuda(v_bits, "v_bits")
+    if v_bits.dtype != torch.int64:                        # (the kernel reads 64-bit elements of contiguous rows)
+        v_bits = (v_bits > 0).to(torch.int64)
+    if v_bits.stride(1) != 1 and v_bits.shape[1] > 1:
+        v_bits = v_bits.contiguous()
     H, T = v_bits.shape
     out = torch.empty(H, dtype=torch.float32, device=v_bits.device)
     check(lib().rdkv_k_budgets(v_bits.data_ptr(), v_bits.stride(0), H, T, int(head_dim),

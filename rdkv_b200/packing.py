@@ -618,7 +618,8 @@ def pack_selected(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Sequence[T
     for k, v, vb, kb in zip(Ks, Vs, v_bits, k_bits):
         if tuple(vb.shape) != (H, T) or tuple(kb.shape) != (H, D) or tuple(k.shape) != (1, H, T, D) or k.shape != v.shape:
             raise ValueError(f"every layer must be [1,{H},{T},{D}] with v_bits [{H},{T}] and k_bits [{H},{D}]")
-    vb, kb = torch.stack(list(v_bits)), torch.stack(list(k_bits))
+    # (the maps go to the kernels by address: of one type, on the layers' device)
+    vb, kb = (torch.stack([m.to(device=Ks[0].device, dtype=torch.int64) for m in maps]) for maps in (v_bits, k_bits))
     parts = _partition_pair(vb.view(L * H, T), kb.view(L * H, D))
     logical = torch.empty(L, dtype=torch.int64, device=vb.device)
     check(lib().rdkv_logical_bits(vb.data_ptr(), kb.data_ptr(), L, H, T, D, logical.data_ptr(), stream_ptr(vb.device)),

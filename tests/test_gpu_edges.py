@@ -190,6 +190,34 @@ def test_unpack_wide_rows(n8):
     assert torch.equal(unpacked(n8), unpacked(128))
 
 
+@pytest.mark.parametrize("dtype", [torch.int16, torch.int32, torch.float32])
+def test_bit_maps_of_other_types_and_strides(dtype):
+    """Maps that are not contiguous 64-bit integers give what the same maps as such give: the bits a packed
+    layer stands for, the layers themselves, the K budgets."""
+    from rdkv_b200 import synth
+    from rdkv_b200.knapsack_solver import k_budgets_from_v_bits
+    from rdkv_b200.packing import pack_selected
+    H, T, g, L = 2, 203, 4, 2
+    K, V, vb, kb = [], [], [], []
+    for i in range(L):
+        k, v = synth.make_kv(H, T, seed=i)
+        K.append(k.cuda()); V.append(v.cuda())
+        vb.append(synth.make_v_bits(H, T, 90, seed=i).to(torch.int64).cuda())
+        kb.append(synth.make_k_bits(H, seed=i).to(torch.int64).cuda())
+
+    def fields(pairs):
+        return [t for pl, v16 in pairs for t in (pl.K_2bit, pl.K_4bit, pl.K_8bit, pl.V_2bit, pl.V_4bit, pl.V_8bit, v16,
+                                                 pl.allocation_v_bits, pl.allocation_k_bits)]
+
+    want, want_bits = pack_selected(K, V, vb, kb, g)
+    budgets = k_budgets_from_v_bits(60, 128, 0.5, vb[0])
+    for change in (lambda m: m.to(dtype), lambda m: m.to(dtype).t().contiguous().t(), lambda m: m.t().contiguous().t()):
+        got, got_bits = pack_selected(K, V, [change(m) for m in vb], [change(m) for m in kb], g)
+        assert torch.equal(got_bits, want_bits)
+        assert all(torch.equal(a, b) for a, b in zip(fields(got), fields(want)))
+        assert torch.equal(k_budgets_from_v_bits(60, 128, 0.5, change(vb[0])), budgets)
+
+
 @pytest.mark.parametrize("tokens,window,g", [(33, 32, 4), (128, 8, 4), (129, 16, 8), (1000, 32, 8), (5000, 5, 3)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_normalised_window_scores(tokens, window, g, causal):
