@@ -659,8 +659,9 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
     tensors; they get tensors of their own, in launches of a few layers each.  ``launch_events``:
     a list that receives two (start, end) pairs of CUDA events per call, around the partition
     launch and around the packing launches (for measurements).  ``k_passes``: 1 = K packed in one pass over the kept
-    rows (held in the shared memory of a cluster of CTAs; raises if they do not fit), 3 = in three
-    (the rows are read twice), 0 = one pass where it fits; the bytes are the same.
+    rows (held in the shared memory of a cluster of CTAs; raises if they do not fit, except for layers with
+    tensors of their own, where it means 0), 3 = in three (the rows are read twice), 0 = one pass where the rows
+    leave room for a second CTA on an SM, else three; the bytes are the same.
     """
     import ctypes as C
     from ._lib import PackJob
@@ -692,7 +693,7 @@ def pack_kv_layers(Ks: Sequence[Tensor], Vs: Sequence[Tensor], v_bits: Tensor, k
     batch = PackedLayerBatch(L)
     uniform = (n2p == n2p[0]).all() and (n4p == n4p[0]).all() and (n8p == n8p[0]).all() and (dk == dk[0]).all()
     if not uniform or int(n2p[0] + n4p[0] + n8p[0]) == 0:
-        done = _pack_exact(Ks, Vs, parts, shape, gqa_factor, build_mask, k_passes, launch_events)
+        done = _pack_exact(Ks, Vs, parts, shape, gqa_factor, build_mask, 3 if k_passes == 3 else 0, launch_events)
         batch._make = lambda i: done[i]
         return batch
     N2P, N4P, N8P, DK = int(n2p[0]), int(n4p[0]), int(n8p[0]), int(dk[0])

@@ -218,6 +218,26 @@ def test_bit_maps_of_other_types_and_strides(dtype):
         assert torch.equal(k_budgets_from_v_bits(60, 128, 0.5, change(vb[0])), budgets)
 
 
+@pytest.mark.parametrize("k_passes", [0, 1, 3])
+def test_pass_choice_for_layers_of_different_shapes(k_passes):
+    """Layers with tensors of their own take every ``k_passes``, also 1 where their rows do not fit a cluster's
+    shared memory; the bytes are the same."""
+    from rdkv_b200 import synth
+    from rdkv_b200.packing import pack_kv, pack_kv_layers
+    H, T, g = 1, 26000, 2
+    Ks, Vs, vbs, kbs = [], [], [], []
+    for i in range(2):
+        K, V = synth.make_kv(H, T, seed=i)
+        Ks.append(K.cuda()); Vs.append(V.cuda())
+        vbs.append(synth.make_v_bits(H, T, 25000, seed=i).cuda())
+        kbs.append(synth.make_k_bits(H, seed=i, mix=((8, 30 + i), (4, 40), (2, 30))).cuda())
+    batch = pack_kv_layers(Ks, Vs, torch.stack(vbs), torch.stack(kbs), g, build_mask=False, k_passes=k_passes)
+    for i, (pl, _) in enumerate(batch):
+        want, _ = pack_kv(Ks[i], Vs[i], vbs[i], kbs[i], g, build_mask=False)
+        for name in ("K_2bit", "K_4bit", "K_8bit", "K_ch_scale", "K_ch_zp"):
+            assert torch.equal(getattr(pl, name), getattr(want, name)), name
+
+
 @pytest.mark.parametrize("tokens,window,g", [(33, 32, 4), (128, 8, 4), (129, 16, 8), (1000, 32, 8), (5000, 5, 3)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_normalised_window_scores(tokens, window, g, causal):
