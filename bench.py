@@ -628,7 +628,8 @@ def run_pack(args, rank, world, device):
                          "traffic": PACK_NCU_TRAFFIC_BYTES, "peak_kind": kind,
                          "kernel": "partition_pair_kernel + pack_v128_batched_kernel + pack_k_onepass_batched_kernel",
                          "kernel_ms": kern_ms, "algorithmic_bytes_per_step": moved},
-            "gpu_launches": 4 * 2 * args.steps, "clocks": sampler.summary()}
+            # the timed steps and the event-timed ones: partition, V pass and K in one pass or three kernels
+            "gpu_launches": (5 if args.k_passes == 3 else 3) * 2 * args.steps, "clocks": sampler.summary()}
     if not args.no_cpu_baseline:
         from oracle import ref_packing as RP
         K, V, vb, kb = Ks[0].cpu().numpy(), Vs[0].cpu().numpy(), v_bits[0].cpu().numpy(), k_bits[0].cpu().numpy()
@@ -752,7 +753,7 @@ def run_alloc(args, rank, world, device):
 
 def run_aux(args, rank, world, device):
     """The small kernels around the hot path, each timed alone on config-3-sized inputs: the
-    decompressor (one launch per layer), the uncompressed-tail kernel, the log-sum-exp combine, block
+    decompressor (one launch per 16 layers), the uncompressed-tail kernel, the log-sum-exp combine, block
     scoring of the blockwise decoder and the token / channel partition.  One step = each of them once."""
     if rank != 0:
         return None
@@ -835,14 +836,14 @@ def run_aux(args, rank, world, device):
         "decode block, three launches: packed zones + tail_attn_partial_kernel + lse_combine_kernel": (
             lambda: packed_decode_attention(q, dtab, out=dout, new_k=new_k, new_v=new_v, n_new=cap - 1, one_launch=False),
             dbytes + tail_bytes),
-        "unpack_layer_kernel": (lambda: unpack_trizone_to_past_kv(cache, head_dim=128),
+        "unpack_layers128_kernel": (lambda: unpack_trizone_to_past_kv(cache, head_dim=128),
                                 L * H * (N * (34 + 67.5) + 2 * N * 128 * 2)),
         "tail_attn_partial_kernel": (lambda: tail_attention_partial(q, new_k, new_v, cap, H),
                                      n_views * H * cap * 128 * 2 * 2),
         "lse_combine_kernel": (lambda: lse_combine(recs), recs.numel() * 4 + recs.shape[0] * 128 * 4),
         "block_score_kernel": (lambda: [_score_block(bq[l], bk[l], num_kv_groups=g, causal=False) for l in range(L)],
                                L * (H * g * 64 + H * 64) * 128 * 2),
-        "partition_kernel": (lambda: (partition_by_bits(vbits, 0), partition_by_bits(kbits, 1)),
+        "partition_pair_kernel": (lambda: (partition_by_bits(vbits, 0), partition_by_bits(kbits, 1)),
                              vbits.numel() * 2 * 3 + kbits.numel() * 2 * 3),
     }
     peak, kind = load_peaks()
@@ -860,7 +861,7 @@ def run_aux(args, rank, world, device):
             "vs_baseline": None, "dtype": "fp16 / u8", "data": "synthetic",
             "config": {"workload": f"aux: decompress {L} config-3 layers; tail attention 128 views x 8 heads x 1024 rows; "
                                    "combine 16384 x 2 records; block scores of 64-token blocks; partition 256 x 32768 maps"},
-            "kernels": out, "peak_kind": kind, "gpu_launches": args.steps * (4 + 1 + 1 + 3 + L + 1 + 1 + L + 2),
+            "kernels": out, "peak_kind": kind, "gpu_launches": args.steps * (4 + 1 + 1 + 3 + (L + 15) // 16 + 1 + 1 + L + 2),
             "clocks": sampler.summary()}
 
 
