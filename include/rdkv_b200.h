@@ -534,7 +534,7 @@ int rdkv_sizeof_pack_job(void);
  * keeps them in shared memory between the extrema and the quantisation; head size 128, and
  * ceil(max_t_k / 8) rows of max_d_pad fp16 values must fit 200 KB, else RDKV_ERR_TOO_LARGE);
  * 3 = extrema pass, parameter pass, quantise pass (the rows are read twice); 0 = one pass where
- * it fits.  Both give the same bytes.  max_k_quads: max over jobs of n_ch2_pad/4 +
+ * it takes up to 110 KB (two CTAs on an SM), else three.  Both give the same bytes.  max_k_quads: max over jobs of n_ch2_pad/4 +
  * ceil(n_ch4_pad/4) + ceil(n_ch8/4) (what a parked row of the one-pass form holds, in 8-byte
  * units), or 0 for the bound max_d_pad/4 + 2. */
 int rdkv_pack_kv_batched(const rdkv_pack_job* jobs, int n_jobs, int H, int D, int max_slots,

@@ -2234,8 +2234,9 @@ extern "C" int rdkv_decode_weighted_sum(const rdkv_layer_view* views, int n_view
   if (n_views > 1) return RDKV_ERR_BAD_ARG;                 // one weight matrix per call
   const int rc = check_fused_args(views, n_views, weights, RDKV_F32, H_q, H_kv, k_row_bytes_max);
   if (rc != RDKV_OK || n_views == 0) return rc;
-  // One view has H_kv units: a CTA each left 140 SMs idle (8 heads x 1792 rows: 30 us).  A unit's rows are cut
-  // into up to 8 chunks (a portable cluster) of at least 128 rows while the chunks fit the chip.
+  // One view has H_kv units, and a CTA each would leave 140 SMs idle.  A unit's rows are cut into up to 8 chunks
+  // (a portable cluster) of at least 128 rows while the chunks fit the chip.  The kernel alone, inputs not in L2, before
+  // and after: 8 heads x 1792 rows 33 -> 18 us, 8 x 2048 35 -> 18.
   int dev = 0, sms = 0, chunks = 1;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     g_last_cuda_error = (int)cudaGetLastError();

@@ -589,7 +589,10 @@ constexpr int PACKK_ROWS = 128;                              // stripe rows per 
 constexpr int PACKK_RPW = PACKK_ROWS / PACKK_WARPS;          // rows per warp and block
 constexpr int PACKK_BPC = 4;                                 // blocks per CTA, at most
 
-// CTAs per head: as few as give every SM two CTAs (three fit), at most one per block
+// CTAs per head: as few as make four for each of the 148 SMs (three are resident at a time), at most one per
+// block.  Quantise kernel of ragged heads x 8, us with four against two per SM: 4 layers x 2048 rows 25 / 29,
+// 8 x 2048 44 / 54, 2 x 8192 45 / 51, 4 x 8192 67 / 67, 1 x 4096 (one CTA per block both ways) 13 / 13; two
+// are the better number for one layer of 8192 rows only, 22 / 20.
 __host__ inline int pack_k_quant_ctas(int t_k, int64_t heads) {
   const int blocks = (t_k + PACKK_ROWS - 1) / PACKK_ROWS;
   const int64_t wanted = (4 * 148 + heads - 1) / heads, least = (blocks + PACKK_BPC - 1) / PACKK_BPC;
@@ -876,8 +879,9 @@ constexpr int KOP_CL = 8;
 constexpr int KOP_WARPS = 8;
 constexpr int KOP_MAX_SMEM = 200 * 1024;
 // By itself the one-pass form is taken where two of its CTAs fit an SM: the gather needs the second one's
-// loads in flight.  (4 layers x 8 heads, device time of the K launches: 4096 rows in 75 KB per CTA 27.7 us
-// against 53.3 in three passes, 32 layers 181 against 267; 8192 rows of 92 channels in 190 KB 166 against 109.)
+// loads in flight.  (4 layers x 8 heads, the K kernels one by one with inputs not in L2: 4096 rows of 64 channels
+// in 75 KB per CTA 29 us against 16 + 6 + 30 in three passes, 32 layers of them 174 against 82 + 7 + 130; 4096 ragged
+// rows in 95 KB 49 against 15 + 7 + 44; 8192 ragged rows in 190 KB 166 against 21 + 7 + 67.)
 constexpr int KOP_AUTO_SMEM = 110 * 1024;
 
 __host__ __device__ inline int kop_rows_per_cta(int t_k) { return (((t_k + KOP_CL - 1) / KOP_CL) + 31) & ~31; }

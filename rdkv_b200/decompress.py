@@ -133,8 +133,8 @@ def _unpack_v_perhead(pl: PackedKVLayer, *, head_dim: int) -> Tensor:
 
 def _fill_view(v: LayerView, pl: PackedKVLayer, V16: Optional[Tensor], rows: int) -> Optional[list]:
     """The fields of ``rdkv_layer_view`` the decompressor reads, straight from a layer whose tensors are
-    ``[1,H_kv,...]`` with contiguous rows (what this library packs); False for any other layer, which takes
-    :func:`rdkv_b200.packing.layer_view`.  Returns the temporaries to keep alive."""
+    ``[1,H_kv,...]`` with contiguous rows (what this library packs).  Returns the temporaries to keep alive; None
+    for any other layer, which takes :func:`rdkv_b200.packing.layer_view`."""
     n2c, n4c, n8c = pl.K_ch_seg_bounds
     v.n_ch2_pad, v.n_ch4_pad, v.n_ch8 = (n2c + 3) // 4 * 4, (n4c + 1) // 2 * 2, n8c
     for name, stride_name, t in (("k2", "k2_head_stride", pl.K_2bit if n2c else None), ("k4", "k4_head_stride", pl.K_4bit if n4c else None),

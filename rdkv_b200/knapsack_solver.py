@@ -4,7 +4,9 @@ Drop-in for the reference's ``knapsack_bit_allocation_batched`` and its scalar
 twin (knapsack_solver.py:39-248): same arguments, same LongTensor result, and
 bit-for-bit the same choices as the reference produces on CPU.  The whole
 multiplier search (lambda_hi doubling, lambda = 0 shortcut, bisection with
-per-row freeze) runs inside one kernel pair, one CTA per row.
+per-row freeze) runs on the GPU in one launch, a warp per short row and a cluster
+of CTAs per long one; a second, small launch does rows again whose doublings the
+batch-wide exit would have cut short.
 """
 from __future__ import annotations
 

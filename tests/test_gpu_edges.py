@@ -1,5 +1,5 @@
 """Prefill kernels at the sizes where they change their way of working: partition (tiles of 256 elements,
-eight in registers, clusters of CTAs), allocator (a warp per short row, clusters and buckets for long ones),
+eight kept in shared memory, clusters of CTAs), allocator (a warp per short row, clusters and buckets for long ones),
 batched packing of layers of different shapes, budgets, unpacking; against the oracle, bit for bit."""
 import numpy as np
 import pytest
